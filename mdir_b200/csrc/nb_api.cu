@@ -198,6 +198,7 @@ int32_t mdrtNbCreate(mdrtNb **out, int32_t device, int64_t particles) {
   cudaMemset(c.sizes, 0, sizeof(int32_t) * NB_SIZE_COUNT);
   cudaMemset(c.status, 0, sizeof(int32_t));
   cudaMemset(c.energy, 0, sizeof(double) * NB_E_SLOTS);
+  cudaStreamSynchronize(nullptr);  // cleared before any stream's use
   // default particle table: no charge, one type of no interaction
   std::vector<double> q(particles, 0.0);
   std::vector<int32_t> t(particles, 0);
@@ -409,7 +410,8 @@ int32_t mdrtNbSetPrunedReach(mdrtNb *ctx, double pruned_distance) {
   if (c.inner_reach > 0.0 && c.built) {
     int64_t key = c.groups_cap * 1000003 + c.list_cap * 7 + c.units_cap;
     if (key != c.inner_key || !c.slab_in) {
-      if (nb_reserve_inner(c)) return MDRT_NB_CUDA_ERROR;
+      if (nb_reserve_inner(c, nullptr)) return MDRT_NB_CUDA_ERROR;
+      CK(cudaStreamSynchronize(nullptr));  // cleared before any stream's pruning
       c.inner_key = key;
     }
   }
@@ -579,7 +581,7 @@ static int32_t nb_force_entry(mdrtNb *ctx, const double *x, const double box[3],
 // The checks of the gradient entries and the adjoint's scratch (allocated
 // here, outside any capture).
 static int32_t nb_gradient_ready(mdrtNb *ctx, const double *x, const double box[3], const double *cotangent,
-                                 int32_t mode, const float *phi, double *dq, double *dtable) {
+                                 int32_t mode, const float *phi, double *dq, double *dtable, void *stream) {
   if (!ctx || !x || !box || !dq || !dtable) return MDRT_NB_INVALID_ARGUMENT;
   if (mode != MDRT_NB_GRAD_PRODUCT && mode != MDRT_NB_GRAD_ENERGY) return MDRT_NB_INVALID_ARGUMENT;
   if (mode == MDRT_NB_GRAD_PRODUCT && !cotangent) return MDRT_NB_INVALID_ARGUMENT;
@@ -594,7 +596,7 @@ static int32_t nb_gradient_ready(mdrtNb *ctx, const double *x, const double box[
   if (c.lj_switch) return MDRT_NB_UNSUPPORTED;
   if (phi && !c.pme.on) return MDRT_NB_INVALID_ARGUMENT;
   CK(cudaSetDevice(c.device));
-  if (nb_adjoint_reserve(c)) return MDRT_NB_CUDA_ERROR;
+  if (nb_adjoint_reserve(c, (cudaStream_t)stream)) return MDRT_NB_CUDA_ERROR;
   return MDRT_NB_OK;
 }
 
@@ -629,7 +631,7 @@ int32_t mdrtNbParameterGradientFrames(mdrtNb *ctx, const double *x, int64_t x_st
                                       void *stream) {
   if (!ctx || count < 0) return MDRT_NB_INVALID_ARGUMENT;
   if (count == 0) return MDRT_NB_OK;
-  int32_t ready = nb_gradient_ready(ctx, x, box, cotangent, mode, potentials, dq, dtable);
+  int32_t ready = nb_gradient_ready(ctx, x, box, cotangent, mode, potentials, dq, dtable, stream);
   if (ready) return ready;
   auto run = [&](cudaStream_t s) -> int32_t {
     if (nb_adjoint_run(ctx->c, x, x_stride, count, box, cotangent, c_stride, mode, potentials, p_stride, dq, dtable,
@@ -732,7 +734,7 @@ int32_t mdrtPmePotentialGrid(mdrtNb *ctx, float *grid, void *stream) {
 int32_t mdrtNbParameterGradientPotential(mdrtNb *ctx, const double *x, const double box[3],
                                          const double *cotangent, int32_t mode, const float *phi, double *dq,
                                          double *dtable, void *stream) {
-  int32_t s = nb_gradient_ready(ctx, x, box, cotangent, mode, phi, dq, dtable);
+  int32_t s = nb_gradient_ready(ctx, x, box, cotangent, mode, phi, dq, dtable, stream);
   if (s) return s;
   if (nb_adjoint_run(ctx->c, x, 0, 1, box, cotangent, 0, mode, phi, 0, dq, dtable, (cudaStream_t)stream))
     return MDRT_NB_CUDA_ERROR;

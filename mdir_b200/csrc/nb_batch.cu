@@ -110,7 +110,8 @@ int32_t mdrtNbBatchCreate(mdrtNbBatch **out, int32_t device, int32_t frames, con
   if (ok) {
     ok = cudaMemcpy(b->atom_frame, af.data(), sizeof(int32_t) * total, cudaMemcpyHostToDevice) == cudaSuccess &&
          cudaMemset(b->frame_energy, 0, sizeof(double) * NB_E_SLOTS * frames) == cudaSuccess &&
-         cudaMemset(b->d_excl_blk0, 0, sizeof(int32_t) * (frames + 1)) == cudaSuccess;
+         cudaMemset(b->d_excl_blk0, 0, sizeof(int32_t) * (frames + 1)) == cudaSuccess &&
+         cudaStreamSynchronize(nullptr) == cudaSuccess;
   }
   b->h_excl_blk0.assign(frames + 1, 0);
   if (!ok) {

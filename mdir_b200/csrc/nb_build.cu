@@ -773,8 +773,10 @@ static int nb_realloc(T *&p, int64_t count) {
 }
 
 // Sizes the buffers for n atoms, the planned columns and bins
-// (c.plan_cols, c.plan_bins) and the list capacity C.
-static int nb_reserve(NbCtx &c, int64_t list_cap) {
+// (c.plan_cols, c.plan_bins) and the list capacity C.  Fresh accumulators
+// are cleared on s, the stream of the launches that use them (the null
+// stream's memset would not come before those of a non-blocking stream).
+static int nb_reserve(NbCtx &c, int64_t list_cap, cudaStream_t s) {
   int64_t n = c.n;
   int64_t cols = c.plan_cols;
   int64_t groups = (n + NB_GROUP - 1) / NB_GROUP + cols;  // at most one partial group a column
@@ -810,8 +812,8 @@ static int nb_reserve(NbCtx &c, int64_t list_cap) {
           nb_realloc(c.pme.tile_sorted, cap * NB_GROUP))
         return -1;
     }
-    NB_CHECK(cudaMemset(c.acc, 0, sizeof(float4) * cap * NB_GROUP));
-    NB_CHECK(cudaMemset(c.acc_fixed, 0, sizeof(unsigned long long) * cap * NB_GROUP * 3));
+    NB_CHECK(cudaMemsetAsync(c.acc, 0, sizeof(float4) * cap * NB_GROUP, s));
+    NB_CHECK(cudaMemsetAsync(c.acc_fixed, 0, sizeof(unsigned long long) * cap * NB_GROUP * 3, s));
     c.groups_cap = cap;
     c.places_cap = cap * NB_GROUP;
   }
@@ -928,7 +930,7 @@ void nb_build_launch_public(NbCtx &c, const double *x, const double box[3], cuda
   nb_build_launch(c, x, box, s);
 }
 
-int nb_reserve_inner(NbCtx &c) {
+int nb_reserve_inner(NbCtx &c, cudaStream_t s) {
   // the inner buffers follow the outer capacities
   int64_t G = c.groups_cap, C = c.list_cap, U = c.units_cap;
   c.slab_in_entries = 0;
@@ -939,7 +941,7 @@ int nb_reserve_inner(NbCtx &c) {
   if (!c.sizes_in) {
     if (cudaMalloc(&c.sizes_in, sizeof(int32_t) * NB_SIZE_COUNT) != cudaSuccess) return -1;
   }
-  cudaMemset(c.sizes_in, 0, sizeof(int32_t) * NB_SIZE_COUNT);
+  if (cudaMemsetAsync(c.sizes_in, 0, sizeof(int32_t) * NB_SIZE_COUNT, s) != cudaSuccess) return -1;
   c.inner_valid = false;
   return 0;
 }
@@ -1052,7 +1054,7 @@ int nb_build_run(NbCtx &c, const double *x, const double box[3], cudaStream_t s)
       return -1;
   }
   for (int attempt = 0; attempt < 8; ++attempt) {
-    if (nb_reserve(c, cap)) return -1;
+    if (nb_reserve(c, cap, s)) return -1;
     nb_build_launch(c, x, box, s);
     NB_CHECK(cudaMemcpyAsync(c.h_sizes, c.sizes, sizeof(int32_t) * NB_SIZE_COUNT,
                              cudaMemcpyDeviceToHost, s));
@@ -1066,7 +1068,7 @@ int nb_build_run(NbCtx &c, const double *x, const double box[3], cudaStream_t s)
       if (c.inner_reach > 0.0) {
         int64_t key = c.groups_cap * 1000003 + c.list_cap * 7 + c.units_cap;
         if (key != c.inner_key || !c.slab_in) {
-          if (nb_reserve_inner(c)) return -1;
+          if (nb_reserve_inner(c, s)) return -1;
           c.inner_key = key;
         }
       }
@@ -1154,7 +1156,7 @@ int nb_grow_lists(NbCtx &c, int64_t longest) {
   int64_t want = (longest + longest / 4 + NB_UNIT - 1) / NB_UNIT * NB_UNIT;
   if (want <= c.list_cap) return 0;
   c.grows++;
-  return nb_reserve(c, want);
+  return nb_reserve(c, want, nullptr);  // the groups stay: nothing is cleared
 }
 
 // ---------------------------------------------------------------------------
@@ -1391,7 +1393,7 @@ int nb_batch_build_run(mdrtNbBatch &b, const double *x, cudaStream_t s) {
   }
   if (!b.frame_units && nb_realloc(b.frame_units, 2 * (int64_t)b.frames)) return -1;
   for (int attempt = 0; attempt < 8; ++attempt) {
-    if (nb_reserve(c, cap)) return -1;
+    if (nb_reserve(c, cap, s)) return -1;
     if (c.groups_cap > b.groups_alloc) {
       if (nb_realloc(b.group_frame, c.groups_cap) || nb_realloc(b.group_L, c.groups_cap)) return -1;
       b.groups_alloc = c.groups_cap;

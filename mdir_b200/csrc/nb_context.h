@@ -283,8 +283,9 @@ void nb_prune_run(NbCtx &c, const double box[3], cudaStream_t s);
 // per-step pruning of the MD step, which needs no conditional node.
 void nb_prune_gated(NbCtx &c, const double box[3], const int *gate, const double *x, double *x_prune,
                     double *prunes, int32_t *unit_counter, cudaStream_t s);
-// Allocates the inner lists to the outer capacities (host, between launches).
-int nb_reserve_inner(NbCtx &c);
+// Allocates the inner lists to the outer capacities (host, between launches);
+// their sizes are cleared on s.
+int nb_reserve_inner(NbCtx &c, cudaStream_t s);
 // Grows the list capacity for lists of up to `longest` entries (+25%), as
 // the count of a build that overflowed asks (host, between launches).
 int nb_grow_lists(NbCtx &c, int64_t longest);
@@ -340,7 +341,7 @@ int nb_pme_run(NbCtx &c, const double box[3], bool energy, bool potential, cudaS
 // dq (f64 [n], atom order) and the type-pair gradient to dtable (f64,
 // ntypes^2 sigma entries then ntypes^2 epsilon entries), each reduced once
 // at the end of the call.  Needs the adjoint scratch (nb_adjoint_reserve).
-int nb_adjoint_reserve(NbCtx &c);
+int nb_adjoint_reserve(NbCtx &c, cudaStream_t s);
 // After a build (host, stream s): the stable partition of each group's
 // entries by whether the partner's type has LJ terms, when the lists are
 // the ones the kernels walk (no pruned reach) and fit the kernel's staging.

@@ -857,7 +857,7 @@ static void md_drop_graph(mdrtMd *m) {
 
 // The integrator's PME buffers when the update gathers (order 4 with a
 // reciprocal sum), sized for the context's grid; none otherwise.
-static int md_pme_buffers(mdrtMd *m) {
+static int md_pme_buffers(mdrtMd *m, cudaStream_t s) {
   NbCtx &c = *m->nb;
   bool want = c.pme.on && c.beta > 0.0 && c.pme.order == 4;
   int64_t pts = want ? (int64_t)c.pme.K[0] * c.pme.K[1] * c.pme.K[2] : 0;
@@ -880,8 +880,8 @@ static int md_pme_buffers(mdrtMd *m) {
   // the grids start empty; each chain empties the grid it spread (the
   // forward plane kernel of the own transforms; with cuFFT the conversion
   // of the fixed-point grid or the spectrum scaling)
-  if (cudaMemset(m->qfixed, 0, sizeof(unsigned long long) * pts) != cudaSuccess ||
-      cudaMemset(m->qgrid, 0, sizeof(float) * pts) != cudaSuccess)
+  if (cudaMemsetAsync(m->qfixed, 0, sizeof(unsigned long long) * pts, s) != cudaSuccess ||
+      cudaMemsetAsync(m->qgrid, 0, sizeof(float) * pts, s) != cudaSuccess)
     return -1;
   m->pme_points = pts;
   return 0;
@@ -1050,6 +1050,7 @@ int32_t mdrtMdCreate(mdrtMd **out, mdrtNb *nb, const double *masses, int64_t nwa
   cudaMemset(m->peak, 0, sizeof(int32_t) * 4);
   cudaMemset(m->flag, 0, sizeof(int) * 4);
   cudaMemset(m->force, 0, sizeof(double) * 3 * c.n);
+  cudaStreamSynchronize(nullptr);  // cleared before any stream's use
   *out = m;
   return MDRT_NB_OK;
 }
@@ -1096,7 +1097,7 @@ int32_t mdrtMdBuild(mdrtMd *m, const double *x, const double box[3], void *strea
     return MDRT_NB_CUDA_ERROR;
   nb_gather_frames(c, x, box, st);
   md_refresh_places(*m, st);
-  if (md_pme_buffers(m)) return MDRT_NB_CUDA_ERROR;
+  if (md_pme_buffers(m, st)) return MDRT_NB_CUDA_ERROR;
   md_after_build<<<blocks_for(3 * m->n, 256), 256, 0, st>>>(3 * m->n, x, m->x_ref, m->thermo, c.sizes, c.status,
                                                             m->peak);
   if (c.inner_reach > 0.0) {

@@ -1312,7 +1312,7 @@ void nb_reduce_energy(NbCtx &c, bool pairs, bool excluded, cudaStream_t s) {
                                     eb, pairs ? 1 : 0, c.energy);
 }
 
-int nb_adjoint_reserve(NbCtx &c) {
+int nb_adjoint_reserve(NbCtx &c, cudaStream_t s) {
   ensure_sm_count();
   // per block of the adjoint kernel, the 2 ntypes^2 type-pair sums
   int width = 2 * c.ntypes * c.ntypes;
@@ -1332,7 +1332,9 @@ int nb_adjoint_reserve(NbCtx &c) {
     c.adj_places = 0;
     if (cudaMalloc(&c.adj_g, sizeof(float4) * c.places_cap) != cudaSuccess) return -1;
     if (cudaMalloc(&c.adj_q, sizeof(double) * c.places_cap) != cudaSuccess) return -1;
-    if (cudaMemset(c.adj_q, 0, sizeof(double) * c.places_cap) != cudaSuccess) return -1;
+    // on the call's stream: a null-stream memset would wait for the work
+    // queued there and could clear sums a side stream's kernels had made
+    if (cudaMemsetAsync(c.adj_q, 0, sizeof(double) * c.places_cap, s) != cudaSuccess) return -1;
     c.adj_places = c.places_cap;
   }
   return 0;

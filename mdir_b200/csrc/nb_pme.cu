@@ -1218,6 +1218,8 @@ int nb_pme_setup(NbCtx &c, int k0, int k1, int k2, int order) {
         cudaMalloc(&P.tile_sorted, sizeof(int32_t) * c.places_cap) != cudaSuccess)
       return -1;
   }
+  // the grids are empty before any stream spreads into them
+  if (cudaStreamSynchronize(nullptr) != cudaSuccess) return -1;
   P.on = true;
   return 0;
 }
