@@ -228,7 +228,7 @@ int32_t mdrtNbDestroy(mdrtNb *ctx) {
   if (ctx->drift_done) cudaEventDestroy(ctx->drift_done);
   nb_free(c.excl_off); nb_free(c.excl); nb_free(c.excl_pairs); nb_free(c.excl_partials);
   nb_free(c.order); nb_free(c.place_of); nb_free(c.shift); nb_free(c.xw);
-  nb_free(c.box_lo); nb_free(c.box_hi); nb_free(c.group_start); nb_free(c.group_col);
+  nb_free(c.group_start); nb_free(c.group_col);
   nb_free(c.slab); nb_free(c.counts); nb_free(c.unit_n); nb_free(c.unit_start); nb_free(c.units);
   nb_free(c.sizes); nb_free(c.status);
   nb_free(c.key); nb_free(c.bin_count); nb_free(c.bin_start); nb_free(c.bin_fill);

@@ -134,7 +134,6 @@ int32_t mdrtNbBatchDestroy(mdrtNbBatch *b) {
   bfree(b->group_frame);
   bfree(b->group_L);
   bfree(b->frame_units);
-  bfree(b->search_scratch);
   bfree(b->excl_blk_frame);
   bfree(b->excl_blk_first);
   bfree(b->excl_frame_end);
@@ -342,7 +341,7 @@ int32_t mdrtNbBatchAutotune(mdrtNbBatch *b, const double *x, double *forces, voi
   CK(cudaEventCreate(&e0));
   CK(cudaEventCreate(&e1));
   float best = 1e30f;
-  int best_w = b->search_warps, best_p = c.pair_blocks_per_sm, best_d = c.staging_depth;
+  int best_w = 4, best_p = c.pair_blocks_per_sm, best_d = c.staging_depth;
   int32_t status = MDRT_NB_OK;
   for (int w : {4, 1}) {
     for (int trial = 0; trial < 8; ++trial) {
@@ -378,10 +377,6 @@ int32_t mdrtNbBatchAutotune(mdrtNbBatch *b, const double *x, double *forces, voi
   b->search_warps = best_w;
   c.pair_blocks_per_sm = best_p;
   c.staging_depth = best_d;
-  if (best_w == 1) {  // a warp a group stages nothing
-    bfree(b->search_scratch);
-    b->search_scratch_entries = 0;
-  }
   drop_graph(b);
   if (choice) {
     choice[0] = best_w;

@@ -10,17 +10,18 @@
 // The B200 design differs from the reference's: the cell sort is a counting
 // sort into columns of about 16 atoms per column-width of height (so a
 // group of 16 consecutive places of a column is close to a cube, with no
-// sorting network); the search screens whole candidate groups against the
-// group's bounding box, 32 candidates a ballot, then tests the 16 x 16
-// pairs of two candidate groups per warp pass with the f32 test; the
-// exclusion partners of the 16 members are sorted in shared memory and
+// sorting network); the search takes a run of places from each column around
+// a group by the z bins of the sort (no candidate's box is read), tests the
+// places against the group's box, 32 or 128 at a time, and those that pass
+// against its 16 members; the exclusion partners of the 16 members are
+// sorted in shared memory and
 // looked up by binary search; and the list of a group is a fixed slab of C
 // entries (grown by the host when a build reports a longer list), so that
 // the units of work come out in group order and every result is
 // deterministic.
 //
 // Kernels (in launch order): nb_keys, scan, nb_scatter, nb_bin_sort,
-// nb_col_groups, scan, nb_group_cols, nb_places, nb_boxes, nb_search,
+// nb_col_groups, scan, nb_group_cols, nb_places, nb_search_t,
 // nb_unit_count, scan, nb_unit_write.
 #include <cmath>
 #include <cstdio>
@@ -151,29 +152,9 @@ __global__ void nb_places(int nsorted_max, const int32_t *__restrict__ bin_start
   order[p] = a;
   place_of[a] = (int32_t)p;
   shift[p] = atom_shift[a];
-  xw[p] = atom_xw[a];
-}
-
-__global__ void nb_boxes(int64_t groups_cap, const int32_t *__restrict__ sizes,
-                         const int32_t *__restrict__ order, const float4 *__restrict__ xw,
-                         float4 *__restrict__ box_lo, float4 *__restrict__ box_hi) {
-  int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= groups_cap || g >= sizes[NB_SIZE_GROUPS]) return;
-  float lo0 = INFINITY, lo1 = INFINITY, lo2 = INFINITY;
-  float hi0 = -INFINITY, hi1 = -INFINITY, hi2 = -INFINITY;
-  for (int u = 0; u < NB_GROUP; ++u) {
-    int64_t p = g * NB_GROUP + u;
-    if (order[p] < 0) continue;
-    float4 v = xw[p];
-    lo0 = fminf(lo0, v.x);
-    lo1 = fminf(lo1, v.y);
-    lo2 = fminf(lo2, v.z);
-    hi0 = fmaxf(hi0, v.x);
-    hi1 = fmaxf(hi1, v.y);
-    hi2 = fmaxf(hi2, v.z);
-  }
-  box_lo[g] = make_float4(lo0, lo1, lo2, 0.f);
-  box_hi[g] = make_float4(hi0, hi1, hi2, 0.f);
+  float4 v = atom_xw[a];
+  v.w = __int_as_float(a);  // the search reads place and atom together
+  xw[p] = v;
 }
 
 // The f32 distance of the pair test, the same for both orders of the pair:
@@ -188,88 +169,116 @@ __device__ __forceinline__ float nb_pair_r2(float4 xa, float4 xb, float sx, floa
 
 struct SearchParams {
   float Lx, Ly, Lz;
-  float bx, cx, cy;  // the tilts of a triclinic cell (tri != 0), else 0
-  int tri;
-  float wx, wy;
-  int Nx, Ny;
+  float bx, cx, cy;  // the tilts of a triclinic cell (TRI), else 0
+  float wx, wy, inv_hz;
+  int Nx, Ny, Nz;
   float R2f;     // (float)(R'^2)
   float Rbox;    // R' plus a margin, for the conservative box and window tests
   int64_t groups_cap;
   int64_t list_cap;
 };
 
+// A coordinate no position comes near: an empty member place lies beyond
+// any reach of every candidate (its square stays finite in f32).
+#define NB_NOWHERE 1e18f
+
 // W warps build the list of one group (W = 1: a warp a group, four groups
-// a block; W = 4: a block a group).  Lanes 0-15 and 16-31 of a warp hold the
-// members; a pass tests two candidate groups, one per half-warp, each lane
-// one candidate place against the 16 members.  With W > 1 the columns of the
-// window are cut into W contiguous shares, each warp stages its entries and
-// the block writes them in warp order, so a list is the same for every W.
-// The staging is shared memory (list_cap entries a warp) without `scratch`;
-// with it, a ring of 64 entries a warp in shared memory whose full runs of
-// 32 go to chunks claimed in the group's row of `scratch` (groups_cap x
-// list_cap entries, the inner slab, which a build invalidates anyway), so
-// that a block needs a few KB, not 4 list_cap x 8 B, and many blocks fit on
-// an SM.
-template <int W, bool BATCH>
+// a block; W = 4: a block a group).
+//
+// The window.  A lane takes one (column, image) of the window around the
+// group's box and finds the run of places of that column that can lie within
+// the reach: the columns are sorted by z bin, so the height the reach leaves
+// at the column's distance in x and y gives the run from two bin starts, with
+// no look at the places.  The runs of 32 such lanes are laid end to end (a
+// warp scan) and cut into chunks of 32 candidates, so no lane waits for the
+// longest run and a column's far places are never read.
+//
+// The tests.  A lane takes one candidate place against the group's box;
+// those that pass wait in a queue in window order, and whole warps of them
+// run the 16 member tests.  With W = 4 a chunk is 128 candidates, the
+// queue is the block's, and counts of the four warps keep the order, so a
+// list is the same for every W.
+//
+// What bounds it: the member tests' arithmetic (16 tests of 8 operations, each
+// rounded once, packed in pairs, for about two thirds of the candidates); a
+// chunk's place loads are issued two chunks at a time.  Reading whole columns of groups, their
+// boxes, then their places one pair of groups at a time took 3,350 µs for the
+// 1.07 M-atom box at 1.0 nm and 27 ms at 1.6 nm; this takes 631 and 1,570.
+template <int W, bool BATCH, bool TRI = false>
 __global__ void __launch_bounds__(128) nb_search_t(SearchParams P0, const NbFrameDev *__restrict__ frames,
                                                    const int32_t *__restrict__ group_frame,
                                                    const int32_t *sizes_in,
                                                    const int32_t *__restrict__ order,
                                                    const float4 *__restrict__ xw,
-                                                   const float4 *__restrict__ box_lo,
-                                                   const float4 *__restrict__ box_hi,
                                                    const int32_t *__restrict__ group_start,
+                                                   const int32_t *__restrict__ bin_start,
                                                    const int32_t *__restrict__ excl_off,
                                                    const int32_t *__restrict__ excl,
                                                    int2 *__restrict__ slab, int32_t *__restrict__ counts,
-                                                   int32_t *sizes, int2 *__restrict__ scratch) {
-  constexpr int GPB = 4 / W;  // groups per block
-  extern __shared__ int2 s_stage[];
-  __shared__ int2 s_ring[W > 1 ? W : 1][64];
-  __shared__ int s_fill;
-  __shared__ int4 s_qi[4][64];    // a warp's queue: place, atom, image code, member bound | same group
-  __shared__ float4 s_qx[4][64];  // and the place's frame
-  __shared__ float4 s_mem[GPB][NB_GROUP];
-  __shared__ int s_atom[GPB][NB_GROUP];
-  __shared__ int s_key[GPB][NB_EXCL_MAX];
-  __shared__ unsigned char s_ku[GPB][NB_EXCL_MAX];
+                                                   int32_t *sizes) {
+  constexpr int GPB = 4 / W;       // groups per block
+  constexpr int CHUNK = 32 * W;    // candidates a step
+  constexpr int QCAP = 2 * CHUNK;  // the queue (a step adds at most CHUNK to fewer than CHUNK)
+  __shared__ float4 s_qx[GPB][QCAP];  // the queue: the place's position, its atom in w
+  __shared__ int2 s_qi[GPB][QCAP];    // and the place and the image code
+  __shared__ float4 s_run[4][32];     // a warp's runs: the image's shift, its code in w
+  __shared__ int2 s_runp[4][32];      // and its first place less its offset, and the offset
+  __shared__ float4 s_mem[GPB][NB_GROUP];  // the members, the atom in w
+  // members m and m + 8 side by side for the packed tests: (x, x', y, y'), (z, z')
+  __shared__ float4 s_mxy[GPB][NB_GROUP / 2];
+  __shared__ float2 s_mz[GPB][NB_GROUP / 2];
+  __shared__ int s_raw[GPB][NB_EXCL_MAX], s_key[GPB][NB_EXCL_MAX];  // exclusions: partner * 16 + member
   __shared__ int s_meta[GPB][4];  // nkeys, wide, kmin, kmax
-  __shared__ int s_count[4];
+  __shared__ int s_kept[W], s_has[W];
   const unsigned FULL = 0xffffffffu;
-  int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  int u = lane & 15, half = lane >> 4;
-  int gi = warp / W, part = warp % W;
-  int64_t g = (int64_t)blockIdx.x * GPB + gi;
-  int ngroups = sizes_in[NB_SIZE_GROUPS];
-  bool live = g < ngroups && g < P0.groups_cap;
-  if (W == 1 && !live) return;
-  // a frame of a batch: its cell, grid, reach and first column
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int u = lane & 15, half = lane >> 4;
+  const int gi = warp / W, part = warp % W;
+  const unsigned below = (1u << lane) - 1u;
+  const int64_t g = (int64_t)blockIdx.x * GPB + gi;
+  // W = 4: the same for the whole block; W = 1: for the warp
+  if (g >= sizes_in[NB_SIZE_GROUPS] || g >= P0.groups_cap) return;
+  auto sync = [&]() {
+    if (W > 1)
+      __syncthreads();
+    else
+      __syncwarp();
+  };
+  // a frame of a batch: its cell, grid, reach, first column and first bin
   SearchParams P = P0;
-  int col0 = 0;
-  if (BATCH && live) {
+  int col0 = 0, bin0 = 0;
+  if (BATCH) {
     const NbFrameDev &F = frames[group_frame[g]];
     P.Lx = F.Lf0;
     P.Ly = F.Lf1;
     P.Lz = F.Lf2;
     P.wx = F.wx;
     P.wy = F.wy;
+    P.inv_hz = F.inv_hz;
     P.Nx = F.Nx;
     P.Ny = F.Ny;
+    P.Nz = F.Nz;
     P.R2f = F.R2f;
     P.Rbox = F.Rbox;
     col0 = F.col0;
+    bin0 = F.bin0;
   }
 
-  // members and the exclusion partners of the members: keys (partner atom,
-  // member), sorted; by the first warp of the group
-  if (live && part == 0) {
-    int64_t pi = g * NB_GROUP + u;
-    int ai = order[pi];
-    float4 xi = xw[pi];
-    if (half == 0) {
-      xi.w = ai >= 0 ? 1.f : 0.f;
-      s_mem[gi][u] = xi;
-      s_atom[gi][u] = ai;
+  // the members and their box, in every warp of the group
+  const int ai = order[g * NB_GROUP + u];
+  float4 xi = ai >= 0 ? xw[g * NB_GROUP + u] : make_float4(NB_NOWHERE, NB_NOWHERE, NB_NOWHERE, 0.f);
+  xi.w = __int_as_float(ai);
+  float3 lo, hi;
+  nb_live_box(xi, ai >= 0, lo, hi);
+  // the exclusion partners of the members: keys (partner atom, member),
+  // sorted; by the first warp of the group
+  if (part == 0) {
+    if (half == 0) s_mem[gi][u] = xi;
+    const float ox = __shfl_sync(FULL, xi.x, lane + 8), oy = __shfl_sync(FULL, xi.y, lane + 8);
+    const float oz = __shfl_sync(FULL, xi.z, lane + 8);
+    if (lane < NB_GROUP / 2) {
+      s_mxy[gi][lane] = make_float4(xi.x, ox, xi.y, oy);
+      s_mz[gi][lane] = make_float2(xi.z, oz);
     }
     int rs = 0, re = 0;
     if (excl_off && half == 0 && ai >= 0) {
@@ -287,39 +296,24 @@ __global__ void __launch_bounds__(128) nb_search_t(SearchParams P0, const NbFram
     bool wide = nkeys > NB_EXCL_MAX;
     if (!wide) {
       int at = incl - cnt;
-      for (int k = 0; k < cnt; ++k) {
-        s_key[gi][at + k] = excl[rs + k];
-        s_ku[gi][at + k] = (unsigned char)u;
-      }
+      for (int k = 0; k < cnt; ++k) s_raw[gi][at + k] = excl[rs + k] * NB_GROUP + u;
     } else if (lane == 0) {
       atomicAdd(&sizes[NB_SIZE_EXCL_WIDE], 1);
     }
     __syncwarp();
     int kmin = INT_MAX, kmax = INT_MIN;
-    if (!wide && nkeys > 0) {
-      // rank sort of the keys by (partner, member, position)
-      int myk[NB_EXCL_MAX / 32];
-      unsigned char myu[NB_EXCL_MAX / 32];
-      int myr[NB_EXCL_MAX / 32];
-      int mine = 0;
-      for (int k = lane; k < nkeys; k += 32, ++mine) {
-        int kv = s_key[gi][k];
-        unsigned char ku = s_ku[gi][k];
+    if (!wide) {
+      // rank sort of the keys (atom numbers stay below 2^26: they fit)
+      for (int k = lane; k < nkeys; k += 32) {
+        const int kv = s_raw[gi][k];
         int r = 0;
         for (int t = 0; t < nkeys; ++t) {
-          int tv = s_key[gi][t];
+          const int tv = s_raw[gi][t];
           r += (tv < kv) || (tv == kv && t < k);
         }
-        myk[mine] = kv;
-        myu[mine] = ku;
-        myr[mine] = r;
-        kmin = min(kmin, kv);
-        kmax = max(kmax, kv);
-      }
-      __syncwarp();
-      for (int m = 0; m < mine; ++m) {
-        s_key[gi][myr[m]] = myk[m];
-        s_ku[gi][myr[m]] = myu[m];
+        s_key[gi][r] = kv;
+        kmin = min(kmin, kv / NB_GROUP);
+        kmax = max(kmax, kv / NB_GROUP);
       }
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) {
@@ -333,288 +327,278 @@ __global__ void __launch_bounds__(128) nb_search_t(SearchParams P0, const NbFram
       s_meta[gi][2] = kmin;
       s_meta[gi][3] = kmax;
     }
-    __syncwarp();
   }
-  const bool chunked = W > 1 && scratch != nullptr;
-  const int chunk_cap = (int)(P.list_cap / 32) + 1;  // chunk offsets a warp
-  int *chunk_at = chunked ? (int *)s_stage + warp * chunk_cap : nullptr;
-  int2 *ring = s_ring[W > 1 ? warp : 0];
-  int rhead = 0, rn = 0, nchunks = 0;  // the ring's first entry and size; chunks written
-  if (chunked && threadIdx.x == 0) s_fill = 0;
-  if (W > 1) __syncthreads();
-  else __syncwarp();
-  int count = 0;
-  int2 *stage = (W > 1 && !chunked) ? s_stage + (size_t)warp * P.list_cap : nullptr;
-  if (live) {
-    int nkeys = s_meta[gi][0];
-    bool wide = s_meta[gi][1] != 0;
-    int kmin = s_meta[gi][2], kmax = s_meta[gi][3];
-    float4 lo = box_lo[g], hi = box_hi[g];
-    NbCell H;
-    H.ax = P.Lx;
-    H.by = P.Ly;
-    H.cz = P.Lz;
-    H.bx = P.bx;
-    H.cx = P.cx;
-    H.cy = P.cy;
-    float ci0 = 0.5f * (lo.x + hi.x), ci1 = 0.5f * (lo.y + hi.y), ci2 = 0.5f * (lo.z + hi.z);
-    float wi0 = 0.5f * (hi.x - lo.x), wi1 = 0.5f * (hi.y - lo.y), wi2 = 0.5f * (hi.z - lo.z);
-    int kx0 = (int)floorf((lo.x - P.Rbox) / P.wx), kx1 = (int)floorf((hi.x + P.Rbox) / P.wx);
-    int ky0 = (int)floorf((lo.y - P.Rbox) / P.wy), ky1 = (int)floorf((hi.y + P.Rbox) / P.wy);
-    int sz0 = (lo.z - P.Rbox < 0.f) ? -1 : 0;
-    int sz1 = (hi.z + P.Rbox >= P.Lz) ? 1 : 0;
-    float Rb2 = P.Rbox * P.Rbox;
-    int nx = kx1 - kx0 + 1, nwin = (ky1 - ky0 + 1) * nx;
-    int w0 = (int)((int64_t)nwin * part / W), w1 = (int)((int64_t)nwin * (part + 1) / W);
+  sync();
+  const int nkeys = s_meta[gi][0];
+  const bool wide = s_meta[gi][1] != 0;
+  const int kmin = s_meta[gi][2], kmax = s_meta[gi][3];
+  NbCell H;
+  H.ax = P.Lx;
+  H.by = P.Ly;
+  H.cz = P.Lz;
+  H.bx = P.bx;
+  H.cx = P.cx;
+  H.cy = P.cy;
+  const float Rb2 = P.Rbox * P.Rbox;
+  int2 *const row = slab + g * P.list_cap;
+  float4 *const qx = s_qx[gi];
+  int2 *const qi = s_qi[gi];
+  int qh = 0, qn = 0;  // the queue's first entry and size (the same in every warp of the group)
+  int count = 0;       // entries written
 
-    // Places of the candidate groups that pass the test against this
-    // group's box wait in a queue of 64 a warp; the member tests then run a
-    // place a lane over 32 of them at once, in queue order (the order of the
-    // window, so the list is the one of testing every place), and no lane
-    // idles on a place that the box test dropped.
-    int4 *qi = s_qi[warp];
-    float4 *qx = s_qx[warp];
-    int qh = 0, qn = 0;  // the queue's first entry and size (warp-uniform)
-    auto drain = [&](int take) {
-      __syncwarp();
-      unsigned mask = 0;
-      int pj = 0, code = 0;
-      if (lane < take) {
-        int4 e = qi[(qh + lane) & 63];
-        float4 xj = qx[(qh + lane) & 63];
-        pj = e.x;
-        int aj = e.y;
-        code = e.z;
-        int uu = e.w & 15;
-        bool same = ((e.w >> 4) & 1) != 0;
-        int sx, sy, sz;
-        nb_decode_image(code, sx, sy, sz);
-        float3 t = nb_lattice_shift(sx, sy, sz, H);
-        float fsx = t.x, fsy = t.y, fsz = t.z;
-#pragma unroll 4
-        for (int m = 0; m < NB_GROUP; ++m) {
-          float4 xm = s_mem[gi][m];
-          int am = s_atom[gi][m];
-          // canonical orientation: A = smaller atom number
-          bool jfirst = aj < am;
-          float4 xa = jfirst ? xj : xm;
-          float4 xb = jfirst ? xm : xj;
-          float sgn = jfirst ? -1.f : 1.f;
-          float r2 = nb_pair_r2(xa, xb, sgn * fsx, sgn * fsy, sgn * fsz);
-          bool ok = (xm.w != 0.f) && (r2 <= P.R2f) && (!same || m < uu);
-          mask |= ok ? (1u << m) : 0u;
-        }
-        if (mask) {
-          if (!wide) {
-            if (nkeys > 0 && aj >= kmin && aj <= kmax) {
-              int lo_i = 0, hi_i = nkeys;
-              while (lo_i < hi_i) {
-                int mid = (lo_i + hi_i) >> 1;
-                if (s_key[gi][mid] < aj) lo_i = mid + 1; else hi_i = mid;
-              }
-              for (int k = lo_i; k < nkeys && s_key[gi][k] == aj; ++k)
-                mask &= ~(1u << s_ku[gi][k]);
-            }
-          } else {
-            unsigned mm = mask;
-            while (mm) {
-              int m = __ffs(mm) - 1;
-              mm &= mm - 1;
-              int am = s_atom[gi][m];
-              for (int k = excl_off[am]; k < excl_off[am + 1]; ++k)
-                if (excl[k] == aj) mask &= ~(1u << m);
-            }
-          }
-        }
+  // The member tests of the first `take` places of the queue, a lane each
+  // (warp `part` takes the part-th 32 of them), in queue order.
+  auto drain = [&](int take) {
+    unsigned mask = 0;
+    int pj = 0, code = 0;
+    const int k = 32 * part + lane;
+    const bool on = k < take;
+    float4 xj = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (on) {
+      int2 e = qi[(qh + k) & (QCAP - 1)];
+      xj = qx[(qh + k) & (QCAP - 1)];
+      pj = e.x;
+      code = e.y;
+    }
+    const int home = nb_image_code(0, 0, 0);
+    int sx, sy, sz;
+    nb_decode_image(on ? code : home, sx, sy, sz);
+    const float3 t = nb_lattice_shift(sx, sy, sz, H);
+    // x_j + s L - x_m, two members at a time in packed f32x2 arithmetic (each
+    // difference, product and sum rounded once, as nb_pair_r2's).  In the
+    // home cell the two orientations of the canonical distance differ in sign
+    // alone, so this is it.  Through an image it is within `slack` of it: what
+    // lies that near the reach is tested again in the canonical orientation.
+    const float ix = __fadd_rn(xj.x, t.x), iy = __fadd_rn(xj.y, t.y), iz = __fadd_rn(xj.z, t.z);
+    const float2 nx = make_float2(-ix, -ix), ny = make_float2(-iy, -iy), nz = make_float2(-iz, -iz);
+    auto tests = [&](float limit) {
+      unsigned in = 0;
+#pragma unroll
+      for (int m = 0; m < NB_GROUP / 2; ++m) {
+        const float4 a = s_mxy[gi][m];
+        const float2 dx = __fadd2_rn(make_float2(a.x, a.y), nx), dy = __fadd2_rn(make_float2(a.z, a.w), ny);
+        const float2 dz = __fadd2_rn(s_mz[gi][m], nz);
+        const float2 r2 = __fadd2_rn(__fadd2_rn(__fmul2_rn(dx, dx), __fmul2_rn(dy, dy)), __fmul2_rn(dz, dz));
+        in |= r2.x <= limit ? (1u << m) : 0u;
+        in |= r2.y <= limit ? (1u << (m + 8)) : 0u;
       }
-      unsigned has = __ballot_sync(FULL, mask != 0);
-      if (chunked) {
-        if (mask)
-          ring[(rhead + rn + __popc(has & ((1u << lane) - 1))) & 63] =
-              make_int2(pj, (int)(mask | ((unsigned)code << 16)));
-        rn += __popc(has);
-        if (rn >= 32) {  // a full run of 32 to a chunk of the group's scratch row
-          __syncwarp();
-          int claim = 0;
-          if (lane == 0) claim = atomicAdd(&s_fill, 32);
-          claim = __shfl_sync(FULL, claim, 0);
-          if (claim + 32 <= P.list_cap) scratch[g * P.list_cap + claim + lane] = ring[(rhead + lane) & 63];
-          if (lane == 0 && nchunks < chunk_cap) chunk_at[nchunks] = claim + 32 <= P.list_cap ? claim : -1;
-          ++nchunks;
-          rhead = (rhead + 32) & 63;
-          rn -= 32;
-          __syncwarp();
-        }
-      } else if (mask) {
-        int at = count + __popc(has & ((1u << lane) - 1));
-        int2 en = make_int2(pj, (int)(mask | ((unsigned)code << 16)));
-        if (at < P.list_cap) {
-          if (W > 1)
-            stage[at] = en;
-          else
-            slab[g * P.list_cap + at] = en;
-        }
-      }
-      count += __popc(has);
-      qh = (qh + take) & 63;
-      qn -= take;
-      __syncwarp();
+      return in;
     };
-
-    // The candidate groups of column c seen through the image T (code):
-    // the box test, then the places that pass the test against this group's
-    // box into the queue.
-    auto visit = [&](int c, float fsx, float fsy, float fsz, int code) {
-      int hb = max(group_start[c], (int)g), he = group_start[c + 1];
-      for (int base = hb; base < he; base += 32) {
-        int hc = base + lane;
-        bool pass = false;
-        if (hc < he) {
-          float4 l2 = box_lo[hc], h2 = box_hi[hc];
-          float d0 = fabsf(0.5f * (l2.x + h2.x) + fsx - ci0) - (wi0 + 0.5f * (h2.x - l2.x));
-          float d1 = fabsf(0.5f * (l2.y + h2.y) + fsy - ci1) - (wi1 + 0.5f * (h2.y - l2.y));
-          float d2 = fabsf(0.5f * (l2.z + h2.z) + fsz - ci2) - (wi2 + 0.5f * (h2.z - l2.z));
-          d0 = fmaxf(d0, 0.f);
-          d1 = fmaxf(d1, 0.f);
-          d2 = fmaxf(d2, 0.f);
-          pass = d0 * d0 + d1 * d1 + d2 * d2 <= Rb2;
+    mask = tests(P.R2f);
+    if (__ballot_sync(FULL, on && code != home) != 0u) {
+      const float slack = 4e-6f * P.Rbox * (H.ax + H.by + H.cz + fabsf(H.bx) + fabsf(H.cx) + fabsf(H.cy));
+      unsigned doubt = tests(P.R2f + slack) & ~tests(P.R2f - slack);
+      if (!on || code == home) doubt = 0;
+      const int aj = __float_as_int(xj.w);
+      while (doubt) {
+        const int m = __ffs(doubt) - 1;
+        doubt &= doubt - 1;
+        const float4 xm = s_mem[gi][m];
+        // canonical orientation: A the smaller atom number, d = (x_B + s L) - x_A
+        const bool jfirst = aj < __float_as_int(xm.w);
+        const float sgn = jfirst ? -1.f : 1.f;
+        const float r2 = nb_pair_r2(jfirst ? xj : xm, jfirst ? xm : xj, sgn * t.x, sgn * t.y, sgn * t.z);
+        mask = r2 <= P.R2f ? mask | (1u << m) : mask & ~(1u << m);
+      }
+    }
+    if (!on) mask = 0;
+    if ((pj >> 4) == (int)g) mask &= (1u << (pj & 15)) - 1u;  // inside the group, each pair once
+    if (mask) {
+      const int aj = __float_as_int(xj.w);
+      if (!wide) {
+        if (nkeys > 0 && aj >= kmin && aj <= kmax) {
+          int lo_i = 0, hi_i = nkeys;
+          while (lo_i < hi_i) {
+            int mid = (lo_i + hi_i) >> 1;
+            if (s_key[gi][mid] < aj * NB_GROUP) lo_i = mid + 1; else hi_i = mid;
+          }
+          for (int e = lo_i; e < nkeys && s_key[gi][e] / NB_GROUP == aj; ++e)
+            mask &= ~(1u << (s_key[gi][e] & (NB_GROUP - 1)));
         }
-        unsigned bits = __ballot_sync(FULL, pass);
-        while (bits) {
-          int c0 = __ffs(bits) - 1;
-          bits &= bits - 1;
-          int c1 = -1;
-          if (bits) {
-            c1 = __ffs(bits) - 1;
-            bits &= bits - 1;
-          }
-          int cand = half ? c1 : c0;
-          bool keep = false;
-          int pj = 0, aj = -1;
-          float4 xj = make_float4(0.f, 0.f, 0.f, 0.f);
-          bool same = false;
-          if (cand >= 0) {
-            int64_t h = base + cand;
-            pj = (int)(h * NB_GROUP + u);
-            aj = order[pj];
-            if (aj >= 0) {
-              xj = xw[pj];
-              same = h == g;
-              // the place against this group's box, with the margin of the window
-              float xs = xj.x + fsx, ys = xj.y + fsy, zs = xj.z + fsz;
-              float gx = fmaxf(fmaxf(lo.x - xs, xs - hi.x), 0.f);
-              float gy = fmaxf(fmaxf(lo.y - ys, ys - hi.y), 0.f);
-              float gz = fmaxf(fmaxf(lo.z - zs, zs - hi.z), 0.f);
-              keep = gx * gx + gy * gy + gz * gz <= Rb2;
-            }
-          }
-          unsigned kb = __ballot_sync(FULL, keep);
-          if (keep) {
-            int at = (qh + qn + __popc(kb & ((1u << lane) - 1))) & 63;
-            qi[at] = make_int4(pj, aj, code, u | (same ? 16 : 0));
-            qx[at] = xj;
-          }
-          qn += __popc(kb);
-          if (qn >= 32) drain(32);
+      } else {
+        unsigned mm = mask;
+        while (mm) {
+          int m = __ffs(mm) - 1;
+          mm &= mm - 1;
+          int am = __float_as_int(s_mem[gi][m].w);
+          for (int e = excl_off[am]; e < excl_off[am + 1]; ++e)
+            if (excl[e] == aj) mask &= ~(1u << m);
         }
       }
-    };
-
-    if (!P.tri) {
-      // orthorhombic: the window of columns around the box, wrapped per axis
-      for (int wi = w0; wi < w1; ++wi) {
-        int ky = ky0 + wi / nx, kx = kx0 + wi % nx;
-        int cy = ((ky % P.Ny) + P.Ny) % P.Ny;
-        int sy = (ky - cy) / P.Ny;
-        int cx = ((kx % P.Nx) + P.Nx) % P.Nx;
-        int sx = (kx - cx) / P.Nx;
-        int c = col0 + cy * P.Nx + cx;
-        if (max(group_start[c], (int)g) >= group_start[c + 1]) continue;
-        for (int sz = sz0; sz <= sz1; ++sz) {
-          float3 t = nb_lattice_shift(sx, sy, sz, H);
-          visit(c, t.x, t.y, t.z, nb_image_code(sx, sy, sz));
-        }
+    }
+    const unsigned has = __ballot_sync(FULL, mask != 0);
+    int at = count + __popc(has & below);
+    if (W > 1) {
+      if (lane == 0) s_has[part] = __popc(has);
+      sync();
+#pragma unroll
+      for (int w = 0; w < W; ++w) {
+        if (w < part) at += s_has[w];
+        count += s_has[w];
       }
     } else {
-      // triclinic: every lattice vector n that can bring a brick position
-      // within the reach of the box (along c, then b, then a), each with the
-      // brick's columns its window cuts; the (image, column) pairs are
-      // shared among the W warps in this order.
-      const float R = P.Rbox;
-      auto each = [&](auto &&fn) {
-        int nc0 = (int)floorf((lo.z - R) / H.cz), nc1 = (int)floorf((hi.z + R) / H.cz);
-        for (int nc = nc0; nc <= nc1; ++nc) {
-          float yc = (float)nc * H.cy, xc = (float)nc * H.cx;
-          int nb0 = (int)floorf((lo.y - R - yc) / H.by), nb1 = (int)floorf((hi.y + R - yc) / H.by);
-          for (int nb = nb0; nb <= nb1; ++nb) {
-            float xb = xc + (float)nb * H.bx;
-            int na0 = (int)floorf((lo.x - R - xb) / H.ax), na1 = (int)floorf((hi.x + R - xb) / H.ax);
-            for (int na = na0; na <= na1; ++na) {
-              float3 t = nb_lattice_shift(na, nb, nc, H);
-              if (hi.z + R - t.z < 0.f || lo.z - R - t.z >= H.cz) continue;
-              int ax0 = max(0, (int)floorf((lo.x - R - t.x) / P.wx));
-              int ax1 = min(P.Nx - 1, (int)floorf((hi.x + R - t.x) / P.wx));
-              int ay0 = max(0, (int)floorf((lo.y - R - t.y) / P.wy));
-              int ay1 = min(P.Ny - 1, (int)floorf((hi.y + R - t.y) / P.wy));
-              if (ax0 > ax1 || ay0 > ay1) continue;
-              fn(na, nb, nc, t, ax0, ax1, ay0, ay1);
-            }
+      count += __popc(has);
+      __syncwarp();
+    }
+    if (mask && at < P.list_cap) row[at] = make_int2(pj, (int)(mask | ((unsigned)code << 16)));
+    qh = (qh + take) & (QCAP - 1);
+    qn -= take;
+  };
+
+  // The places that pass the test against the group's box into the queue, in
+  // candidate order; a full chunk of the queue is drained.
+  auto push = [&](bool valid, int p, float4 xj, float4 run) {
+    bool keep = false;
+    if (valid) {
+      const float xs = xj.x + run.x, ys = xj.y + run.y, zs = xj.z + run.z;
+      const float gx = fmaxf(fmaxf(lo.x - xs, xs - hi.x), 0.f);
+      const float gy = fmaxf(fmaxf(lo.y - ys, ys - hi.y), 0.f);
+      const float gz = fmaxf(fmaxf(lo.z - zs, zs - hi.z), 0.f);
+      keep = gx * gx + gy * gy + gz * gz <= Rb2;
+    }
+    const unsigned kb = __ballot_sync(FULL, keep);
+    int at = qh + qn + __popc(kb & below);
+    if (W > 1) {
+      if (lane == 0) s_kept[part] = __popc(kb);
+      sync();
+#pragma unroll
+      for (int w = 0; w < W; ++w) {
+        if (w < part) at += s_kept[w];
+        qn += s_kept[w];
+      }
+    } else {
+      qn += __popc(kb);
+    }
+    if (keep) {
+      qx[at & (QCAP - 1)] = xj;
+      qi[at & (QCAP - 1)] = make_int2(p, __float_as_int(run.w));
+    }
+    sync();  // the queue is written (and s_kept read) before the drain and the next push
+    if (qn >= CHUNK) drain(CHUNK);
+  };
+
+  // 32 columns of the window (one a lane; `on` marks those in it) seen
+  // through the image t: their runs of places, laid end to end.
+  auto columns = [&](bool on, int cx, int cy, float3 t, int code) {
+    int p0 = 0, len = 0;
+    if (on) {
+      const int c = col0 + cy * P.Nx + cx;
+      const int gs = group_start[c];
+      if (group_start[c + 1] > (int)g) {
+        // the column's distance from the group's box in x and y leaves the
+        // height the reach can take in z (the margin of Rbox covers the
+        // rounding of the columns' edges)
+        const float x0 = cx * P.wx + t.x, y0 = cy * P.wy + t.y;
+        const float dx = fmaxf(fmaxf(x0 - hi.x, lo.x - (x0 + P.wx)), 0.f);
+        const float dy = fmaxf(fmaxf(y0 - hi.y, lo.y - (y0 + P.wy)), 0.f);
+        const float z2 = Rb2 - dx * dx - dy * dy;
+        if (z2 >= 0.f) {
+          const float zr = sqrtf(z2);
+          const float z0 = lo.z - zr - t.z, z1 = hi.z + zr - t.z;
+          if (z1 >= 0.f && z0 <= P.Lz) {
+            // the bins as nb_keys takes them: (int)(z inv_hz) does not decrease with z
+            const int k0 = min(max((int)(z0 * P.inv_hz), 0), P.Nz - 1);
+            const int k1 = min(max((int)(z1 * P.inv_hz), 0), P.Nz - 1);
+            const int b = bin0 + (c - col0) * P.Nz;
+            const int s0 = bin_start[b];
+            p0 = max(gs * NB_GROUP + bin_start[b + k0] - s0, (int)g * NB_GROUP);
+            const int p1 = min(gs * NB_GROUP + bin_start[b + k1 + 1] - s0, (int)P.groups_cap * NB_GROUP);
+            len = max(p1 - p0, 0);
           }
         }
-      };
-      int total = 0;
-      each([&](int, int, int, float3, int ax0, int ax1, int ay0, int ay1) {
-        total += (ax1 - ax0 + 1) * (ay1 - ay0 + 1);
-      });
-      int t0 = (int)((int64_t)total * part / W), t1 = (int)((int64_t)total * (part + 1) / W);
-      int at = 0;
-      each([&](int na, int nb, int nc, float3 t, int ax0, int ax1, int ay0, int ay1) {
-        int nxw = ax1 - ax0 + 1, cnt = nxw * (ay1 - ay0 + 1);
-        int lo_i = max(t0 - at, 0), hi_i = min(t1 - at, cnt);
-        for (int k = lo_i; k < hi_i; ++k) {
-          int c = col0 + (ay0 + k / nxw) * P.Nx + ax0 + k % nxw;
-          if (max(group_start[c], (int)g) >= group_start[c + 1]) continue;
-          visit(c, t.x, t.y, t.z, nb_image_code(na, nb, nc));
-        }
-        at += cnt;
-      });
+      }
     }
-    if (qn > 0) drain(qn);
-  }
-  if (W == 1) {
-    if (lane == 0) {
-      counts[g] = count;
-      atomicMax(&sizes[NB_SIZE_LONGEST], count);
-      if (count > P.list_cap) atomicOr(&sizes[NB_SIZE_OVERFLOW], 2);
+    const unsigned full = __ballot_sync(FULL, len > 0);
+    if (full == 0u) return;
+    int incl = len;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      int y = __shfl_up_sync(FULL, incl, o);
+      if (lane >= o) incl += y;
     }
-    return;
-  }
-  if (lane == 0) s_count[warp] = count;
-  __syncthreads();
-  if (!live) return;
-  int at = 0, total = 0;
-  for (int w = gi * W; w < gi * W + W; ++w) {
-    if (w < warp) at += s_count[w];
-    total += s_count[w];
-  }
-  if (chunked) {
-    // this warp's chunks in the order written, then what its ring holds
-    for (int k = 0; k < nchunks && k < chunk_cap; ++k) {
-      int from = chunk_at[k];
-      int to = at + 32 * k + lane;
-      if (from >= 0 && to < P.list_cap) slab[g * P.list_cap + to] = scratch[g * P.list_cap + from + lane];
+    const int total = __shfl_sync(FULL, incl, 31), runs = __popc(full);
+    __syncwarp();
+    if (len > 0) {
+      const int r = __popc(full & below);
+      s_run[warp][r] = make_float4(t.x, t.y, t.z, __int_as_float(code));
+      s_runp[warp][r] = make_int2(p0 - (incl - len), incl - len);
     }
-    int to = at + 32 * nchunks + lane;
-    if (lane < rn && to < P.list_cap) slab[g * P.list_cap + to] = ring[(rhead + lane) & 63];
+    __syncwarp();
+    const int off = lane < runs ? s_runp[warp][lane].y : INT_MAX;  // the lane-th run's offset
+    // candidate t0 + lane: its run is the last that starts at or before it
+    auto find = [&](int t0, bool &valid, int &p, float4 &run) {
+      const bool in = off > t0 && off < t0 + 32;
+      const unsigned starts = __reduce_or_sync(FULL, in ? 1u << (off - t0) : 0u);
+      const int first = __popc(__ballot_sync(FULL, off <= t0)) - 1;
+      const int k = (first < 0 ? 0 : first) + __popc(starts & ((2u << lane) - 1u));
+      valid = t0 + lane < total;
+      p = 0;
+      run = s_run[warp][k & 31];
+      if (valid) p = s_runp[warp][k].x + t0 + lane;
+    };
+    for (int t0 = 32 * part; t0 - 32 * part < total; t0 += 2 * CHUNK) {
+      bool va, vb;
+      int pa, pb;
+      float4 ra, rb;
+      find(t0, va, pa, ra);
+      find(t0 + CHUNK, vb, pb, rb);
+      const float4 xa = va ? xw[pa] : make_float4(0.f, 0.f, 0.f, 0.f);
+      const float4 xb = vb ? xw[pb] : make_float4(0.f, 0.f, 0.f, 0.f);
+      push(va, pa, xa, ra);
+      if (t0 - 32 * part + CHUNK < total) push(vb, pb, xb, rb);
+    }
+  };
+
+  if (!TRI) {
+    // orthorhombic: the window of columns around the box, wrapped per axis,
+    // each with the images in z that its height cuts
+    const int kx0 = (int)floorf((lo.x - P.Rbox) / P.wx), kx1 = (int)floorf((hi.x + P.Rbox) / P.wx);
+    const int ky0 = (int)floorf((lo.y - P.Rbox) / P.wy), ky1 = (int)floorf((hi.y + P.Rbox) / P.wy);
+    const int sz0 = (lo.z - P.Rbox < 0.f) ? -1 : 0;
+    const int sz1 = (hi.z + P.Rbox >= P.Lz) ? 1 : 0;
+    const int nz = sz1 - sz0 + 1, nx = kx1 - kx0 + 1, nwin = (ky1 - ky0 + 1) * nx * nz;
+    for (int base = 0; base < nwin; base += 32) {
+      const int s = base + lane, wi = s / nz;
+      const int ky = ky0 + wi / nx, kx = kx0 + wi % nx;
+      const int cy = ((ky % P.Ny) + P.Ny) % P.Ny, cx = ((kx % P.Nx) + P.Nx) % P.Nx;
+      const int sx = (kx - cx) / P.Nx, sy = (ky - cy) / P.Ny, sz = sz0 + s % nz;
+      columns(s < nwin, cx, cy, nb_lattice_shift(sx, sy, sz, H), nb_image_code(sx, sy, sz));
+    }
   } else {
-    int keep = (int)min((int64_t)count, P.list_cap);
-    for (int i = lane; i < keep; i += 32)
-      if (at + i < P.list_cap) slab[g * P.list_cap + at + i] = stage[i];
+    // triclinic: every lattice vector n that can bring a brick position
+    // within the reach of the box (along c, then b, then a), each with the
+    // brick's columns its window cuts
+    const float R = P.Rbox;
+    const int nc0 = (int)floorf((lo.z - R) / H.cz), nc1 = (int)floorf((hi.z + R) / H.cz);
+    for (int nc = nc0; nc <= nc1; ++nc) {
+      const float yc = (float)nc * H.cy, xc = (float)nc * H.cx;
+      const int nb0 = (int)floorf((lo.y - R - yc) / H.by), nb1 = (int)floorf((hi.y + R - yc) / H.by);
+      for (int nb = nb0; nb <= nb1; ++nb) {
+        const float xb = xc + (float)nb * H.bx;
+        const int na0 = (int)floorf((lo.x - R - xb) / H.ax), na1 = (int)floorf((hi.x + R - xb) / H.ax);
+        for (int na = na0; na <= na1; ++na) {
+          const float3 t = nb_lattice_shift(na, nb, nc, H);
+          if (hi.z + R - t.z < 0.f || lo.z - R - t.z >= H.cz) continue;
+          const int ax0 = max(0, (int)floorf((lo.x - R - t.x) / P.wx));
+          const int ax1 = min(P.Nx - 1, (int)floorf((hi.x + R - t.x) / P.wx));
+          const int ay0 = max(0, (int)floorf((lo.y - R - t.y) / P.wy));
+          const int ay1 = min(P.Ny - 1, (int)floorf((hi.y + R - t.y) / P.wy));
+          if (ax0 > ax1 || ay0 > ay1) continue;
+          const int nx = ax1 - ax0 + 1, nwin = nx * (ay1 - ay0 + 1);
+          for (int base = 0; base < nwin; base += 32) {
+            const int s = base + lane;
+            columns(s < nwin, ax0 + s % nx, ay0 + s / nx, t, nb_image_code(na, nb, nc));
+          }
+        }
+      }
+    }
   }
+  sync();  // every warp is past the last drain's counts
+  if (qn > 0) drain(qn);
   if (part == 0 && lane == 0) {
-    counts[g] = total;
-    atomicMax(&sizes[NB_SIZE_LONGEST], total);
-    if (total > P.list_cap) atomicOr(&sizes[NB_SIZE_OVERFLOW], 2);
+    counts[g] = count;
+    atomicMax(&sizes[NB_SIZE_LONGEST], count);
+    if (count > P.list_cap) atomicOr(&sizes[NB_SIZE_OVERFLOW], 2);
   }
 }
 
@@ -799,7 +783,7 @@ static int nb_reserve(NbCtx &c, int64_t list_cap, cudaStream_t s) {
   if (regroup) {
     int64_t cap = groups + groups / 4 + 16;
     if (nb_realloc(c.order, cap * NB_GROUP) || nb_realloc(c.shift, cap * NB_GROUP) ||
-        nb_realloc(c.xw, cap * NB_GROUP) || nb_realloc(c.box_lo, cap) || nb_realloc(c.box_hi, cap) ||
+        nb_realloc(c.xw, cap * NB_GROUP) ||
         nb_realloc(c.group_col, cap) || nb_realloc(c.counts, cap) || nb_realloc(c.unit_n, cap) ||
         nb_realloc(c.unit_start, cap + 1) || nb_realloc(c.xq, cap * NB_GROUP) ||
         nb_realloc(c.xq_lo, cap * NB_GROUP) ||
@@ -856,6 +840,15 @@ static void nb_allow_smem(K kernel, size_t bytes, size_t (&configured)[NB_MAX_DE
   }
 }
 
+// Four warps a group (else one) for a system of this many groups: with one
+// warp each, fewer groups leave the GPU's warp slots empty and a group's
+// chunks come one after the other (23,550 atoms at 1.0 nm: 31 µs with four,
+// 45 with one; at 1.7 nm 74 and 134); with more, the block's waits cost more
+// than they bring (192,000 atoms: 179 and 128; at 1.6 nm 396 and 315;
+// 1.07 M: 965 and 631).  72,000 atoms are even (72 and 65).
+#define NB_SEARCH_FOUR_GROUPS 4000
+static bool nb_search_four(int64_t groups) { return groups < NB_SEARCH_FOUR_GROUPS; }
+
 // Launches one build on `s`. Returns 0; the sizes are left in c.sizes (device).
 static void nb_build_launch(NbCtx &c, const double *x, const double box[3], cudaStream_t s) {
   const NbGrid &G = c.grid;
@@ -879,8 +872,6 @@ static void nb_build_launch(NbCtx &c, const double *x, const double box[3], cuda
   nb_places<<<blocks_for(n, 256), 256, 0, s>>>((int)n, c.bin_start, nbins, c.sorted, c.key, G.Nz,
                                               c.group_start, c.places_cap, c.atom_xw, c.atom_shift,
                                               c.order, c.place_of, c.shift, c.xw);
-  nb_boxes<<<blocks_for(c.groups_cap, 128), 128, 0, s>>>(c.groups_cap, c.sizes, c.order, c.xw,
-                                                        c.box_lo, c.box_hi);
   SearchParams P;
   P.Lx = (float)box[0];
   P.Ly = (float)box[1];
@@ -888,11 +879,12 @@ static void nb_build_launch(NbCtx &c, const double *x, const double box[3], cuda
   P.bx = (float)c.tilt[0];
   P.cx = (float)c.tilt[1];
   P.cy = (float)c.tilt[2];
-  P.tri = nb_triclinic(c) ? 1 : 0;
   P.wx = G.wx;
   P.wy = G.wy;
+  P.inv_hz = 1.0f / G.hz;
   P.Nx = G.Nx;
   P.Ny = G.Ny;
+  P.Nz = G.Nz;
   // the widening: 3e-6 of the sum of the diagonal and the tilts' magnitudes
   double span = box[0] + box[1] + box[2] + fabs(c.tilt[0]) + fabs(c.tilt[1]) + fabs(c.tilt[2]);
   double Rw = c.reach + 3e-6 * span;
@@ -900,23 +892,12 @@ static void nb_build_launch(NbCtx &c, const double *x, const double box[3], cuda
   P.Rbox = (float)(Rw + 2e-5 * span + 1e-6);
   P.groups_cap = c.groups_cap;
   P.list_cap = c.list_cap;
-  // four warps a group staging in chunks of the inner slab when it is there
-  // (a dual list), else in shared memory when that fits, else one warp
-  bool chunked = c.slab_in && c.slab_in_entries >= c.groups_cap * c.list_cap;
-  size_t stage = chunked ? sizeof(int) * 4 * (size_t)(c.list_cap / 32 + 1) : sizeof(int2) * 4 * (size_t)c.list_cap;
-  if (stage <= 200 * 1024) {
-    static size_t configured[NB_MAX_DEVICES] = {};
-    nb_allow_smem(nb_search_t<4, false>, stage, configured);
-    nb_search_t<4, false><<<(int)c.groups_cap, 128, stage, s>>>(P, nullptr, nullptr, c.sizes, c.order, c.xw,
-                                                                c.box_lo, c.box_hi, c.group_start, c.excl_off,
-                                                                c.excl, c.slab, c.counts, c.sizes,
-                                                                chunked ? c.slab_in : nullptr);
-  } else {
-    nb_search_t<1, false><<<blocks_for(c.groups_cap, 4), 128, 0, s>>>(P, nullptr, nullptr, c.sizes, c.order, c.xw,
-                                                                      c.box_lo, c.box_hi, c.group_start,
-                                                                      c.excl_off, c.excl, c.slab, c.counts,
-                                                                      c.sizes, nullptr);
-  }
+  const bool four = nb_search_four((n + NB_GROUP - 1) / NB_GROUP);
+  const int blocks = four ? (int)c.groups_cap : blocks_for(c.groups_cap, 4);
+  auto kernel = nb_triclinic(c) ? (four ? nb_search_t<4, false, true> : nb_search_t<1, false, true>)
+                                : (four ? nb_search_t<4, false> : nb_search_t<1, false>);
+  kernel<<<blocks, 128, 0, s>>>(P, nullptr, nullptr, c.sizes, c.order, c.xw, c.group_start, c.bin_start, c.excl_off,
+                                c.excl, c.slab, c.counts, c.sizes);
   nb_unit_count<<<blocks_for(c.groups_cap, 256), 256, 0, s>>>(c.groups_cap, c.sizes, c.counts,
                                                              c.list_cap, c.unit_n);
   nb_scan(c.unit_n, c.unit_start, (int)c.groups_cap, nullptr, c.scan_scratch, s);
@@ -1244,7 +1225,9 @@ __global__ void nb_batch_places(int nsorted_max, const int32_t *__restrict__ bin
   order[p] = a;
   place_of[a] = (int32_t)p;
   shift[p] = atom_shift[a];
-  xw[p] = atom_xw[a];
+  float4 v = atom_xw[a];
+  v.w = __int_as_float(a);  // the search reads place and atom together
+  xw[p] = v;
 }
 
 __global__ void nb_batch_group_frames(int64_t groups_cap, const int32_t *__restrict__ sizes,
@@ -1347,30 +1330,17 @@ static void nb_batch_build_launch(mdrtNbBatch &b, const double *x, cudaStream_t 
   nb_batch_places<<<blocks_for(n, 256), 256, 0, s>>>((int)n, c.bin_start, nbins, c.sorted, b.atom_col,
                                                     b.col_frame, b.frames_dev, c.group_start, c.places_cap,
                                                     c.atom_xw, c.atom_shift, c.order, c.place_of, c.shift, c.xw);
-  nb_boxes<<<blocks_for(c.groups_cap, 128), 128, 0, s>>>(c.groups_cap, c.sizes, c.order, c.xw, c.box_lo,
-                                                        c.box_hi);
   nb_batch_group_frames<<<blocks_for(c.groups_cap, 256), 256, 0, s>>>(c.groups_cap, c.sizes, c.group_col,
                                                                      b.col_frame, b.frames_dev, b.group_frame,
                                                                      b.group_L);
   SearchParams P = {};
   P.groups_cap = c.groups_cap;
   P.list_cap = c.list_cap;
-  // four warps a group stage in chunks of the batch's scratch rows
-  bool chunked = b.search_scratch && b.search_scratch_entries >= c.groups_cap * c.list_cap;
-  size_t stage = chunked ? sizeof(int) * 4 * (size_t)(c.list_cap / 32 + 1) : sizeof(int2) * 4 * (size_t)c.list_cap;
-  if (b.search_warps == 4 && stage <= 200 * 1024) {
-    static size_t configured[NB_MAX_DEVICES] = {};
-    nb_allow_smem(nb_search_t<4, true>, stage, configured);
-    nb_search_t<4, true><<<(int)c.groups_cap, 128, stage, s>>>(P, b.frames_dev, b.group_frame, c.sizes, c.order,
-                                                               c.xw, c.box_lo, c.box_hi, c.group_start, c.excl_off,
-                                                               c.excl, c.slab, c.counts, c.sizes,
-                                                               chunked ? b.search_scratch : nullptr);
-  } else {
-    nb_search_t<1, true><<<blocks_for(c.groups_cap, 4), 128, 0, s>>>(P, b.frames_dev, b.group_frame, c.sizes,
-                                                                     c.order, c.xw, c.box_lo, c.box_hi,
-                                                                     c.group_start, c.excl_off, c.excl, c.slab,
-                                                                     c.counts, c.sizes, nullptr);
-  }
+  const bool four = b.search_warps ? b.search_warps == 4 : nb_search_four((n + NB_GROUP - 1) / NB_GROUP);
+  const int blocks = four ? (int)c.groups_cap : blocks_for(c.groups_cap, 4);
+  auto kernel = four ? nb_search_t<4, true> : nb_search_t<1, true>;
+  kernel<<<blocks, 128, 0, s>>>(P, b.frames_dev, b.group_frame, c.sizes, c.order, c.xw, c.group_start, c.bin_start,
+                                c.excl_off, c.excl, c.slab, c.counts, c.sizes);
   nb_unit_count<<<blocks_for(c.groups_cap, 256), 256, 0, s>>>(c.groups_cap, c.sizes, c.counts, c.list_cap,
                                                              c.unit_n);
   nb_scan(c.unit_n, c.unit_start, (int)c.groups_cap, nullptr, c.scan_scratch, s);
@@ -1397,11 +1367,6 @@ int nb_batch_build_run(mdrtNbBatch &b, const double *x, cudaStream_t s) {
     if (c.groups_cap > b.groups_alloc) {
       if (nb_realloc(b.group_frame, c.groups_cap) || nb_realloc(b.group_L, c.groups_cap)) return -1;
       b.groups_alloc = c.groups_cap;
-    }
-    if (b.search_warps == 4 && b.search_scratch_entries < c.groups_cap * c.list_cap) {
-      b.search_scratch_entries = 0;
-      if (nb_realloc(b.search_scratch, c.groups_cap * c.list_cap)) return -1;
-      b.search_scratch_entries = c.groups_cap * c.list_cap;
     }
     nb_batch_build_launch(b, x, s);
     NB_CHECK(cudaMemcpyAsync(c.h_sizes, c.sizes, sizeof(int32_t) * NB_SIZE_COUNT, cudaMemcpyDeviceToHost, s));

@@ -86,8 +86,7 @@ struct NbCtx {
   int64_t units_cap = 0;
   int32_t *order = nullptr, *place_of = nullptr;
   char4 *shift = nullptr;  // per place
-  float4 *xw = nullptr;    // per place, f32 wrapped at the build
-  float4 *box_lo = nullptr, *box_hi = nullptr;  // per group
+  float4 *xw = nullptr;    // per place, f32 wrapped at the build, the atom's number in w
   int32_t *group_start = nullptr;  // per column + 1
   int32_t *group_col = nullptr;    // per group
   int2 *slab = nullptr;            // groups_cap * list_cap entries
@@ -122,7 +121,7 @@ struct NbCtx {
   bool inner_valid = false;
   int64_t inner_key = -1;  // the outer capacities the inner buffers were sized for
   int2 *slab_in = nullptr;
-  int64_t slab_in_entries = 0;  // the allocation of slab_in (the search stages in it)
+  int64_t slab_in_entries = 0;  // the allocation of slab_in
   int32_t *counts_in = nullptr;
   int32_t *unit_n_in = nullptr, *unit_start_in = nullptr;
   int2 *units_in = nullptr;
@@ -233,8 +232,6 @@ struct mdrtNbBatch {
   float4 *group_L = nullptr;      // per group: the frame's cell
   int64_t groups_alloc = 0, cols_alloc = 0;
   int32_t *frame_units = nullptr; // per frame: first unit, one past the last
-  int2 *search_scratch = nullptr; // the search's chunks with four warps a group (groups_cap x list_cap)
-  int64_t search_scratch_entries = 0;
   std::vector<double> h_boxes;    // frames x 3 of the last build
   // excluded pairs: blocks of 256 pairs that never straddle two frames
   int32_t *excl_blk_frame = nullptr, *excl_blk_first = nullptr, *excl_frame_end = nullptr;
@@ -259,7 +256,7 @@ struct mdrtNbBatch {
   int32_t *d_excl_blk0 = nullptr, *d_conv_blk0 = nullptr;
   // energies: frames x NB_E_SLOTS (device) and a pinned mirror
   double *frame_energy = nullptr, *h_frame_energy = nullptr;
-  int search_warps = 4;  // tuning: warps a group of the search (1 or 4)
+  int search_warps = 0;  // tuning: warps a group of the search (1 or 4; 0: by the number of groups)
   // the force evaluation as a CUDA graph
   cudaGraphExec_t exec = nullptr;
   cudaGraph_t graph = nullptr;
