@@ -190,14 +190,14 @@ int32_t mdrtNbCreate(mdrtNb **out, int32_t device, int64_t particles) {
   if (cudaMalloc(&c.sizes, sizeof(int32_t) * NB_SIZE_COUNT) != cudaSuccess ||
       cudaMallocHost(&c.h_sizes, sizeof(int32_t) * NB_SIZE_COUNT) != cudaSuccess ||
       cudaMalloc(&c.status, sizeof(int32_t)) != cudaSuccess ||
-      cudaMalloc(&c.energy, sizeof(double) * NB_E_SLOTS) != cudaSuccess ||
+      cudaMalloc(&c.energy, sizeof(double) * (NB_E_SLOTS + 1)) != cudaSuccess ||
       cudaMallocHost(&c.h_energy, sizeof(double) * NB_E_SLOTS) != cudaSuccess) {
     mdrtNbDestroy(ctx);
     return MDRT_NB_CUDA_ERROR;
   }
   cudaMemset(c.sizes, 0, sizeof(int32_t) * NB_SIZE_COUNT);
   cudaMemset(c.status, 0, sizeof(int32_t));
-  cudaMemset(c.energy, 0, sizeof(double) * NB_E_SLOTS);
+  cudaMemset(c.energy, 0, sizeof(double) * (NB_E_SLOTS + 1));
   cudaStreamSynchronize(nullptr);  // cleared before any stream's use
   // default particle table: no charge, one type of no interaction
   std::vector<double> q(particles, 0.0);

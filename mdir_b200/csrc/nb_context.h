@@ -109,7 +109,7 @@ struct NbCtx {
   unsigned long long *acc_fixed = nullptr;  // 3 per place, deterministic mode
   double *unit_partials = nullptr;       // 8 doubles per unit
   double *excl_partials = nullptr;       // 8 doubles per block of the excluded kernel
-  double *energy = nullptr;              // device results: see NbEnergySlot
+  double *energy = nullptr;              // device results: see NbEnergySlot; then the sums' block counter
   double *h_energy = nullptr;            // pinned mirror
   NbPme pme;
   bool built = false;
@@ -172,6 +172,10 @@ enum NbEnergySlot {
   NB_W_REC = 10,   // 6 entries
   NB_E_SLOTS = 16
 };
+
+// The counters of finished blocks of the energy sums (zero between launches),
+// behind the slots: the pairs' and the reciprocal sum's, which may run at once.
+inline unsigned int *nb_done_blocks(const NbCtx &c) { return (unsigned int *)(c.energy + NB_E_SLOTS); }
 
 // The launches of one frames call kept as a CUDA graph (nb_api.cu): the
 // key is the call's arguments followed by the bytes of the context it ran

@@ -30,6 +30,7 @@
 
 #include "nb_context.h"
 #include "nb_prune.cuh"
+#include "nb_sum.cuh"
 
 #define NB_MAX_TYPES 32
 
@@ -783,49 +784,31 @@ __global__ void nb_finish(int64_t places, const int32_t *__restrict__ sizes,
   }
 }
 
-// Fixed-order sums of per-unit (and per-block) partials: one block, each
-// thread a strided run of rows, then a tree.
-__global__ void nb_sum_partials(const double *__restrict__ unit_partials,
-                                const int32_t *__restrict__ sizes, int64_t units_cap,
-                                const double *__restrict__ excl_partials, int excl_blocks,
-                                int do_pairs, double *__restrict__ energy) {
-  __shared__ double s[256][8];
-  double v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  double w[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  if (do_pairs) {
-    int64_t nunits = min((int64_t)sizes[NB_SIZE_UNITS], units_cap);
-    for (int64_t u = threadIdx.x; u < nunits; u += blockDim.x)
-      for (int k = 0; k < 8; ++k) v[k] += unit_partials[u * 8 + k];
-  }
-  for (int64_t b = threadIdx.x; b < excl_blocks; b += blockDim.x)
-    for (int k = 0; k < 8; ++k) w[k] += excl_partials[b * 8 + k];
-  // pairs: lj, coul, W(6); excluded: e, W(6): combine W of both in slots
-  for (int k = 0; k < 8; ++k) s[threadIdx.x][k] = v[k];
+// The sums of the units' and the excluded blocks' partials into the energy
+// slots: the rows' tiles by nb_tile_rows (tiles [0, unit_tiles) of the
+// units, the rest of the excluded blocks), the tiles by the last block.
+__global__ void __launch_bounds__(256) nb_sum_partials(double *__restrict__ unit_partials,
+                                                       const int32_t *__restrict__ sizes, int64_t units_cap,
+                                                       int unit_tiles, double *__restrict__ excl_partials,
+                                                       int excl_blocks, int do_pairs, double *__restrict__ energy,
+                                                       unsigned int *done) {
+  __shared__ double s[256];
+  const int64_t nunits = do_pairs ? min((int64_t)sizes[NB_SIZE_UNITS], units_cap) : 0;
+  const int tile = blockIdx.x;
+  if (tile < unit_tiles)
+    nb_tile_rows<8>(unit_partials, nunits, tile, s);
+  else
+    nb_tile_rows<8>(excl_partials, excl_blocks, tile - unit_tiles, s);
+  if (!nb_last_block(done)) return;
+  double pv = nb_sum_tiles<8>(unit_partials, nunits, s);
+  double xv = nb_sum_tiles<8>(excl_partials, excl_blocks, s);
+  // pairs: lj, coul, W(6); excluded: e, W(6)
+  const int c = threadIdx.x;
+  if (c < 2 && do_pairs) energy[c == 0 ? NB_E_LJ : NB_E_COUL] = pv;
+  if (c == 0 && excl_blocks > 0) energy[NB_E_EXCL] = xv;
+  if (c < 8) s[c] = xv;
   __syncthreads();
-  for (int stride = blockDim.x / 2; stride > 0; stride >>= 1) {
-    if ((int)threadIdx.x < stride)
-      for (int k = 0; k < 8; ++k) s[threadIdx.x][k] += s[threadIdx.x + stride][k];
-    __syncthreads();
-  }
-  double pv[8];
-  for (int k = 0; k < 8; ++k) pv[k] = s[0][k];
-  __syncthreads();
-  for (int k = 0; k < 8; ++k) s[threadIdx.x][k] = w[k];
-  __syncthreads();
-  for (int stride = blockDim.x / 2; stride > 0; stride >>= 1) {
-    if ((int)threadIdx.x < stride)
-      for (int k = 0; k < 8; ++k) s[threadIdx.x][k] += s[threadIdx.x + stride][k];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    if (do_pairs) {
-      energy[NB_E_LJ] = pv[0];
-      energy[NB_E_COUL] = pv[1];
-    }
-    if (excl_blocks > 0) energy[NB_E_EXCL] = s[0][0];
-    for (int k = 0; k < 6; ++k)
-      energy[NB_W_PAIR + k] = (do_pairs ? pv[2 + k] : 0.0) + (excl_blocks > 0 ? s[0][1 + k] : 0.0);
-  }
+  if (c >= 2 && c < 8) energy[NB_W_PAIR + c - 2] = (do_pairs ? pv : 0.0) + (excl_blocks > 0 ? s[c - 1] : 0.0);
 }
 
 // ---------------------------------------------------------------------------
@@ -1308,8 +1291,10 @@ void nb_finish_forces(NbCtx &c, double *forces, int accumulate, cudaStream_t s) 
 void nb_reduce_energy(NbCtx &c, bool pairs, bool excluded, cudaStream_t s) {
   int eb = (excluded && c.n_excl_pairs > 0 && c.beta != 0.0) ? blocks_for(c.n_excl_pairs, 256) : 0;
   bool inner = c.inner_reach > 0.0 && c.inner_valid;
-  nb_sum_partials<<<1, 256, 0, s>>>(c.unit_partials, inner ? c.sizes_in : c.sizes, c.units_cap, c.excl_partials,
-                                    eb, pairs ? 1 : 0, c.energy);
+  int ut = pairs ? (int)((c.units_cap + NB_SUM_TILE - 1) / NB_SUM_TILE) : 0;
+  int et = (eb + NB_SUM_TILE - 1) / NB_SUM_TILE;
+  nb_sum_partials<<<std::max(1, ut + et), 256, 0, s>>>(c.unit_partials, inner ? c.sizes_in : c.sizes, c.units_cap, ut,
+                                                       c.excl_partials, eb, pairs ? 1 : 0, c.energy, nb_done_blocks(c));
 }
 
 int nb_adjoint_reserve(NbCtx &c, cudaStream_t s) {

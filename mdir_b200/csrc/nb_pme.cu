@@ -28,6 +28,7 @@
 #include "nb_fft.cuh"
 #include "nb_scan.cuh"
 #include "nb_spline.cuh"
+#include "nb_sum.cuh"
 
 namespace {
 
@@ -319,22 +320,14 @@ __global__ void __launch_bounds__(256) nb_convolve(ConvParams C, const float *__
   }
 }
 
-__global__ void nb_pme_sum(const double *__restrict__ partials, int nblocks, double *__restrict__ energy) {
-  __shared__ double s[256][7];
-  double v[7] = {0, 0, 0, 0, 0, 0, 0};
-  for (int b = threadIdx.x; b < nblocks; b += blockDim.x)
-    for (int k = 0; k < 7; ++k) v[k] += partials[(int64_t)b * 7 + k];
-  for (int k = 0; k < 7; ++k) s[threadIdx.x][k] = v[k];
-  __syncthreads();
-  for (int stride = blockDim.x / 2; stride > 0; stride >>= 1) {
-    if ((int)threadIdx.x < stride)
-      for (int k = 0; k < 7; ++k) s[threadIdx.x][k] += s[threadIdx.x + stride][k];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    energy[NB_E_REC] = s[0][0];
-    for (int k = 0; k < 6; ++k) energy[NB_W_REC + k] = s[0][1 + k];
-  }
+// The sums of the convolution blocks' energies and virials into the slots.
+__global__ void __launch_bounds__(224) nb_pme_sum(double *__restrict__ partials, int nblocks,
+                                                  double *__restrict__ energy, unsigned int *done) {
+  __shared__ double s[224];
+  nb_tile_rows<7>(partials, nblocks, blockIdx.x, s);
+  if (!nb_last_block(done)) return;
+  const double v = nb_sum_tiles<7>(partials, nblocks, s);
+  if (threadIdx.x < 7) energy[threadIdx.x == 0 ? NB_E_REC : NB_W_REC + threadIdx.x - 1] = v;
 }
 
 // ---------------------------------------------------------------------------
@@ -1284,6 +1277,11 @@ static int nb_pme_table(NbCtx &c, const double box[3], cudaStream_t s) {
   return 0;
 }
 
+static void nb_pme_sums(NbCtx &c, int rows, cudaStream_t s) {
+  nb_pme_sum<<<(rows + NB_SUM_TILE - 1) / NB_SUM_TILE, 224, 0, s>>>(c.pme.partials, rows, c.energy,
+                                                                   nb_done_blocks(c) + 1);
+}
+
 int nb_pme_run(NbCtx &c, const double box[3], bool energy, bool potential, cudaStream_t s) {
   NbPme &P = c.pme;
   if (!P.on) return 0;
@@ -1318,14 +1316,14 @@ int nb_pme_run(NbCtx &c, const double box[3], bool energy, bool potential, cudaS
     if (nb_fft_convolve(P, P.grid, c.deterministic ? P.fixed : nullptr, P.spec, P.grid, P.influence, energy, C,
                         P.partials, nullptr, s))
       return -3;
-    if (energy) nb_pme_sum<<<1, 256, 0, s>>>(P.partials, (int)nb_fft_column_blocks(P.K), c.energy);
+    if (energy) nb_pme_sums(c, (int)nb_fft_column_blocks(P.K), s);
   } else {
     cufftSetStream(P.fwd, s);
     cufftSetStream(P.bwd, s);
     if (cufftExecR2C(P.fwd, P.grid, (cufftComplex *)P.spec) != CUFFT_SUCCESS) return -3;
     if (energy) {
       nb_convolve<true><<<blocks_for(half, 256), 256, 0, s>>>(C, P.moduli, P.spec, P.partials);
-      nb_pme_sum<<<1, 256, 0, s>>>(P.partials, P.conv_blocks, c.energy);
+      nb_pme_sums(c, P.conv_blocks, s);
     } else {
       if (nb_pme_table(c, box, s)) return -1;
       nb_scale_spectrum<<<blocks_for(half, 256), 256, 0, s>>>(half, P.influence, P.spec, nullptr, 0, nullptr);
