@@ -253,6 +253,7 @@ int32_t mdrtNbSetParticles(mdrtNb *ctx, const double *charges, const int32_t *ty
   for (int64_t i = 0; i < c.n; ++i)
     if (types[i] < 0 || types[i] >= ntypes || !std::isfinite(charges[i])) return MDRT_NB_INVALID_ARGUMENT;
   c.h_q.assign(charges, charges + c.n);
+  const bool same_types = (int64_t)c.h_type.size() == c.n && std::equal(c.h_type.begin(), c.h_type.end(), types);
   c.h_type.assign(types, types + c.n);
   c.h_lj.resize((size_t)ntypes * ntypes);
   c.h_c6.resize((size_t)ntypes * ntypes);
@@ -301,6 +302,7 @@ int32_t mdrtNbSetParticles(mdrtNb *ctx, const double *charges, const int32_t *ty
       if (epsilon[a * ntypes + b] != 0.0) on[a] = 1;
   for (int a = 0; a < ntypes; ++a) mask |= on[a] ? (1u << a) : 0u;
   CK(cudaMemcpy(c.lj_on, on, sizeof(on), cudaMemcpyHostToDevice));
+  if (c.lj_mask != mask || !same_types) c.lj_part_build = -1;  // the lists in force are ordered by the types before
   c.lj_mask = mask;
   CK(cudaMemcpy(c.ljf, factors.data(), sizeof(float2) * ntypes, cudaMemcpyHostToDevice));
   CK(cudaMemcpy(c.sigeps, se.data(), sizeof(float2) * ntypes * ntypes, cudaMemcpyHostToDevice));
@@ -499,7 +501,6 @@ static int32_t nb_build_entry(mdrtNb *ctx, const double *x, int64_t n, const dou
   CK(cudaSetDevice(c.device));
   cudaStream_t st = (cudaStream_t)stream;
   if (nb_build_run(c, x, box, st)) return MDRT_NB_CUDA_ERROR;
-  if (nb_lj_partition_run(c, st)) return MDRT_NB_CUDA_ERROR;
   for (int k = 0; k < 3; ++k) c.tilt_built[k] = c.tilt[k];
   if (!c.x_build) CK(cudaMalloc(&c.x_build, sizeof(double) * 3 * c.n));
   CK(cudaMemcpyAsync(c.x_build, x, sizeof(double) * 3 * c.n, cudaMemcpyDeviceToDevice, st));

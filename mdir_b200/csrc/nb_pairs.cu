@@ -995,45 +995,6 @@ __global__ void nb_scatter_place_values(int64_t places, const int32_t *__restric
   }
 }
 
-// The stable partition of each group's list by the partner's LJ terms: the
-// entries whose partner's type has any, then the others, each in their
-// order; counts_lj[g] gets the number of the first.  One warp a group, its
-// entries staged in shared memory (list_cap of them).
-__global__ void __launch_bounds__(32) nb_lj_partition(const int32_t *__restrict__ sizes, int64_t list_cap,
-                                                      const int32_t *__restrict__ counts, int2 *__restrict__ slab,
-                                                      const int32_t *__restrict__ order,
-                                                      const int32_t *__restrict__ type,
-                                                      const int32_t *__restrict__ lj_on,
-                                                      int32_t *__restrict__ counts_lj) {
-  extern __shared__ int2 s_e[];
-  int64_t g = blockIdx.x;
-  if (g >= sizes[NB_SIZE_GROUPS]) return;
-  int lane = threadIdx.x;
-  int cnt = (int)min((int64_t)counts[g], list_cap);
-  int2 *row = slab + g * list_cap;
-  for (int e = lane; e < cnt; e += 32) s_e[e] = row[e];
-  __syncwarp();
-  auto lj = [&](int e) {
-    int a = order[s_e[e].x];
-    return a >= 0 && lj_on[type[a]] != 0;
-  };
-  int nlj = 0;
-  for (int e0 = 0; e0 < cnt; e0 += 32) nlj += __popc(__ballot_sync(0xffffffffu, e0 + lane < cnt && lj(e0 + lane)));
-  int pl = 0, pn = nlj;
-  unsigned below = (1u << lane) - 1u;
-  for (int e0 = 0; e0 < cnt; e0 += 32) {
-    int e = e0 + lane;
-    bool in = e < cnt;
-    bool f = in && lj(e);
-    unsigned bl = __ballot_sync(0xffffffffu, f);
-    unsigned bn = __ballot_sync(0xffffffffu, in && !f);
-    if (in) row[f ? pl + __popc(bl & below) : pn + __popc(bn & below)] = s_e[e];
-    pl += __popc(bl);
-    pn += __popc(bn);
-  }
-  if (lane == 0) counts_lj[g] = nlj;
-}
-
 // The excluded pairs, u = -f q_i q_j erf(beta r)/r, in f64 and atom order.
 // MODE 0: G_q[i] += h f q_j X, X = d/dr [erf(beta r)/r]; MODE 1: G_q[i] -= f q_j erf(beta r)/r.
 template <int MODE>
@@ -1322,38 +1283,6 @@ int nb_adjoint_reserve(NbCtx &c, cudaStream_t s) {
     if (cudaMemsetAsync(c.adj_q, 0, sizeof(double) * c.places_cap, s) != cudaSuccess) return -1;
     c.adj_places = c.places_cap;
   }
-  return 0;
-}
-
-int nb_lj_partition_run(NbCtx &c, cudaStream_t s) {
-  c.lj_part_build = -1;
-  size_t stage = sizeof(int2) * (size_t)c.list_cap;
-  if (c.inner_reach > 0.0 || !c.lj_on || c.groups_cap <= 0 || c.list_cap <= 0 || stage > 227 * 1024) return 0;
-  if (stage > 48 * 1024) {
-    // the shared-memory opt-in for this list capacity (once per device and size)
-    static size_t configured[64] = {};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev < 0 || dev >= 64) return 0;
-    if (configured[dev] < stage) {
-      if (cudaFuncSetAttribute(nb_lj_partition, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)stage) !=
-          cudaSuccess)
-        return -1;
-      configured[dev] = stage;
-    }
-  }
-  if (c.counts_lj_cap < c.groups_cap) {
-    if (c.counts_lj) cudaFree(c.counts_lj);
-    c.counts_lj = nullptr;
-    c.counts_lj_cap = 0;
-    if (cudaMalloc(&c.counts_lj, sizeof(int32_t) * c.groups_cap) != cudaSuccess) return -1;
-    c.counts_lj_cap = c.groups_cap;
-  }
-  nb_lj_partition<<<(unsigned)c.groups_cap, 32, stage, s>>>(c.sizes, c.list_cap, c.counts, c.slab, c.order, c.type,
-                                                            c.lj_on, c.counts_lj);
-  if (cudaGetLastError() != cudaSuccess) return -1;
-  c.lj_part_build = c.builds;
-  c.lj_part_mask = c.lj_mask;
   return 0;
 }
 

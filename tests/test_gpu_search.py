@@ -103,3 +103,38 @@ def test_one_and_four_warps_a_group_give_the_same_lists(cuda):
     # the same lists entry for entry: the pair energies, summed unit by unit, are the same bits
     for term in ("lj", "coulomb"):
         np.testing.assert_array_equal(lists[0][term], lists[1][term])
+
+
+@pytest.mark.parametrize("waters,reach", [(300, 1.0), (1200, 1.0), (1200, 1.6), (2671, 1.2)])
+@pytest.mark.parametrize("seldom", [False, True])
+def test_lj_partners_first_is_the_stable_partition(cuda, waters, reach, seldom):
+    """Without a pruned reach a group's entries of a partner with LJ terms come
+    first, each part in the order found (the lists of a context with a pruned
+    reach); `seldom`: one atom in 30 has them, so the part that moves down
+    overlaps where it lies in a row that is more than half full."""
+    from mdir_b200 import NonbondedTerm, systems
+    from mdir_b200 import _lib as Lb
+    s = systems.tip3p(waters=waters, seed=9)
+    types = np.asarray(s["types"]).copy()
+    if seldom:
+        types[:] = 1
+        types[::30] = 0
+    x = torch.tensor(s["positions"], device="cuda")
+    rows = []
+    for dual in (True, False):
+        t = NonbondedTerm(len(s["charges"]))
+        t.set_particles(s["charges"], types, s["sigma"], s["epsilon"])
+        t.set_exclusions(pairs=s["excluded_pairs"])
+        t.set_interaction(s["cutoff"], min(reach, 0.99 * float(s["box"][0])), s["beta"])
+        if dual:
+            t.set_pruned_reach(0.95)
+        sizes = t.build(x, s["box"])
+        G, cap = sizes[6], t.info()["list_capacity"]
+        e = t.buffer(Lb.SLOT_ENTRIES, np.int32, 2)[: G * cap].reshape(G, cap, 2)
+        c = t.buffer(Lb.SLOT_COUNTS, np.int32)[:G]
+        order = t.buffer(Lb.SLOT_ORDER, np.int32)
+        rows.append([e[g, : c[g]].copy() for g in range(G)])
+        t.close()
+    for found, first in zip(*rows):
+        lj = types[order[found[:, 0]]] == 0
+        np.testing.assert_array_equal(np.concatenate([found[lj], found[~lj]]), first)
