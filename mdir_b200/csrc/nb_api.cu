@@ -228,15 +228,15 @@ int32_t mdrtNbDestroy(mdrtNb *ctx) {
   if (ctx->drift_done) cudaEventDestroy(ctx->drift_done);
   nb_free(c.excl_off); nb_free(c.excl); nb_free(c.excl_pairs); nb_free(c.excl_partials);
   nb_free(c.order); nb_free(c.place_of); nb_free(c.shift); nb_free(c.xw);
-  nb_free(c.group_start); nb_free(c.group_col);
-  nb_free(c.slab); nb_free(c.counts); nb_free(c.unit_n); nb_free(c.unit_start); nb_free(c.units);
+  nb_free(c.group_start);
+  nb_free(c.slab); nb_free(c.counts); nb_free(c.unit_start); nb_free(c.units);
   nb_free(c.sizes); nb_free(c.status);
-  nb_free(c.key); nb_free(c.bin_count); nb_free(c.bin_start); nb_free(c.bin_fill);
-  nb_free(c.sorted); nb_free(c.col_groups); nb_free(c.scan_scratch);
+  nb_free(c.key); nb_free(c.bin_count); nb_free(c.bin_start); nb_free(c.rank);
+  nb_free(c.sorted); nb_free(c.scan_scratch);
   nb_free(c.atom_xw); nb_free(c.atom_shift);
   nb_free(c.xq); nb_free(c.xq_lo); nb_free(c.typ_p); nb_free(c.acc); nb_free(c.acc_fixed);
   nb_free(c.unit_partials); nb_free(c.energy);
-  nb_free(c.slab_in); nb_free(c.counts_in); nb_free(c.unit_n_in); nb_free(c.unit_start_in);
+  nb_free(c.slab_in); nb_free(c.counts_in); nb_free(c.unit_start_in);
   nb_free(c.units_in); nb_free(c.sizes_in); nb_free(c.one);
   if (c.h_sizes) cudaFreeHost(c.h_sizes);
   if (c.h_energy) cudaFreeHost(c.h_energy);

@@ -129,7 +129,6 @@ int32_t mdrtNbBatchDestroy(mdrtNbBatch *b) {
   if (b->nb) nb_batch_pme_release(*b);
   bfree(b->frames_dev);
   bfree(b->atom_frame);
-  bfree(b->atom_col);
   bfree(b->col_frame);
   bfree(b->group_frame);
   bfree(b->group_L);

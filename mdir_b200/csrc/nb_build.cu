@@ -20,9 +20,8 @@
 // the units of work come out in group order and every result is
 // deterministic.
 //
-// Kernels (in launch order): nb_keys, scan, nb_scatter, nb_bin_sort,
-// nb_col_groups, scan, nb_group_cols, nb_places, nb_search_t,
-// nb_unit_count, scan, nb_unit_write.
+// Kernels (in launch order): nb_keys, scan, nb_scatter, nb_columns,
+// nb_places, nb_search_t, nb_unit_blocks, nb_unit_write.
 #include <cmath>
 #include <cstdio>
 
@@ -44,9 +43,8 @@ namespace {
 __global__ void nb_keys(int64_t n, const double *__restrict__ x, double Lx, double Ly, double Lz,
                         double bx, double cx, double cy,
                         int Nx, int Ny, int Nz, float inv_wx, float inv_wy, float inv_hz,
-                        int32_t *__restrict__ key, int32_t *__restrict__ bin_count,
-                        float4 *__restrict__ atom_xw, char4 *__restrict__ atom_shift,
-                        int32_t *__restrict__ sizes) {
+                        int32_t *__restrict__ key, int32_t *__restrict__ rank, int32_t *__restrict__ bin_count,
+                        float4 *__restrict__ atom_xw, char4 *__restrict__ atom_shift) {
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   double v0 = x[3 * i], v1 = x[3 * i + 1], v2 = x[3 * i + 2];
@@ -66,8 +64,7 @@ __global__ void nb_keys(int64_t n, const double *__restrict__ x, double Lx, doub
   }
   if (!ok) {
     key[i] = Nx * Ny * Nz;  // the bin of the positions that have no key
-    atomicAdd(&bin_count[Nx * Ny * Nz], 1);
-    atomicAdd(&sizes[NB_SIZE_NAN], 1);
+    rank[i] = atomicAdd(&bin_count[Nx * Ny * Nz], 1);
     atom_xw[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     atom_shift[i] = make_char4(0, 0, 0, 0);
     return;
@@ -78,62 +75,65 @@ __global__ void nb_keys(int64_t n, const double *__restrict__ x, double Lx, doub
   int kz = min(max((int)(w2 * inv_hz), 0), Nz - 1);
   int k = (ky * Nx + kx) * Nz + kz;
   key[i] = k;
-  atomicAdd(&bin_count[k], 1);
+  rank[i] = atomicAdd(&bin_count[k], 1);
   atom_xw[i] = make_float4(w0, w1, w2, 1.f);
   atom_shift[i] = make_char4((signed char)S0, (signed char)S1, (signed char)S2, 0);
 }
 
-__global__ void nb_scatter(int64_t n, const int32_t *__restrict__ key,
-                           const int32_t *__restrict__ bin_start, int32_t *__restrict__ bin_fill,
-                           int32_t *__restrict__ sorted) {
+// The atoms of each bin, in the order they came (nb_places orders them).
+__global__ void nb_scatter(int64_t n, const int32_t *__restrict__ key, const int32_t *__restrict__ rank,
+                           const int32_t *__restrict__ bin_start, int32_t *__restrict__ sorted) {
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  int k = key[i];
-  int at = bin_start[k] + atomicAdd(&bin_fill[k], 1);
-  sorted[at] = (int32_t)i;
+  sorted[bin_start[key[i]] + rank[i]] = (int32_t)i;
 }
 
-// Each bin's atoms by number, so that the order does not depend on the
-// threads (bins hold about half an atom on average).
-__global__ void nb_bin_sort(int nbins, const int32_t *__restrict__ bin_start,
-                            int32_t *__restrict__ sorted) {
-  int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= nbins) return;
-  int s = bin_start[b], e = bin_start[b + 1];
-  for (int i = s + 1; i < e; ++i) {
-    int v = sorted[i];
-    int j = i - 1;
-    while (j >= s && sorted[j] > v) {
-      sorted[j + 1] = sorted[j];
-      --j;
+// The columns' groups, in one block: a thread a column counts its groups of
+// 16 places and a scan gives their first groups, a block's threads of columns
+// at a time (one pass up to 1,024).  Clears the build's sizes and counts the
+// positions with no key (the bin past the grid).  With `frames` (a batch),
+// column c is of frame col_frame[c].
+template <bool BATCH>
+__global__ void __launch_bounds__(1024) nb_columns(int ncol, int Nz, int nbins, const int32_t *__restrict__ bin_start,
+                                                   const NbFrameDev *__restrict__ frames,
+                                                   const int32_t *__restrict__ col_frame, int64_t groups_cap,
+                                                   int32_t *__restrict__ group_start, int32_t *__restrict__ sizes) {
+  __shared__ int sw[32];
+  int before = 0;
+  for (int c0 = 0; c0 < ncol; c0 += blockDim.x) {
+    const int c = c0 + threadIdx.x;
+    int groups = 0;
+    if (c < ncol) {
+      int b0 = c * Nz, nz = Nz;
+      if (BATCH) {
+        const NbFrameDev &F = frames[col_frame[c]];
+        nz = F.Nz;
+        b0 = F.bin0 + (c - F.col0) * nz;
+      }
+      groups = (bin_start[b0 + nz] - bin_start[b0] + NB_GROUP - 1) / NB_GROUP;
     }
-    sorted[j + 1] = v;
+    int total;
+    const int first = before + nb_block_exclusive_scan(groups, sw, total);
+    before += total;
+    if (c < ncol) group_start[c] = first;
+  }
+  if (threadIdx.x == 0) {
+    group_start[ncol] = before;
+    for (int k = 0; k < NB_SIZE_COUNT; ++k) sizes[k] = 0;
+    sizes[NB_SIZE_GROUPS] = before;
+    sizes[NB_SIZE_PLACES] = before * NB_GROUP;
+    sizes[NB_SIZE_NAN] = bin_start[nbins + 1] - bin_start[nbins];
+    sizes[NB_SIZE_OVERFLOW] = before > groups_cap ? 1 : 0;
   }
 }
 
-__global__ void nb_col_groups(int ncol, int Nz, const int32_t *__restrict__ bin_start,
-                              int32_t *__restrict__ col_groups) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= ncol) return;
-  int nc = bin_start[(c + 1) * Nz] - bin_start[c * Nz];
-  col_groups[c] = (nc + NB_GROUP - 1) / NB_GROUP;
-}
-
-__global__ void nb_group_cols(int ncol, const int32_t *__restrict__ group_start, int64_t groups_cap,
-                              int32_t *__restrict__ group_col, int32_t *__restrict__ sizes) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c == 0) {
-    int g = group_start[ncol];
-    sizes[NB_SIZE_GROUPS] = g;
-    sizes[NB_SIZE_PLACES] = g * NB_GROUP;
-    if (g > groups_cap) atomicOr(&sizes[NB_SIZE_OVERFLOW], 1);
-  }
-  if (c >= ncol) return;
-  for (int g = group_start[c]; g < group_start[c + 1] && g < groups_cap; ++g) group_col[g] = c;
-}
-
+// The places, a thread an atom of the bin order: within its bin (half an
+// atom on average) an atom comes after those of a smaller number, so that the
+// order does not depend on the threads.  With `frames`, the columns of a batch.
+template <bool BATCH>
 __global__ void nb_places(int nsorted_max, const int32_t *__restrict__ bin_start, int nvalid_bins,
                           const int32_t *__restrict__ sorted, const int32_t *__restrict__ key, int Nz,
+                          const NbFrameDev *__restrict__ frames, const int32_t *__restrict__ atom_frame,
                           const int32_t *__restrict__ group_start, int64_t places_cap,
                           const float4 *__restrict__ atom_xw, const char4 *__restrict__ atom_shift,
                           const int32_t *__restrict__ type, const int32_t *__restrict__ lj_on,
@@ -141,15 +141,22 @@ __global__ void nb_places(int nsorted_max, const int32_t *__restrict__ bin_start
                           char4 *__restrict__ shift, float4 *__restrict__ xw) {
   int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= nsorted_max) return;
-  int nvalid = bin_start[nvalid_bins];
-  int a = sorted[s];
-  if (s >= nvalid) {  // positions with no key are in no group
+  const int a = sorted[s], k = key[a];
+  if (k >= nvalid_bins) {  // positions with no key are in no group
     place_of[a] = -1;
     return;
   }
-  int c = key[a] / Nz;
-  int rank = s - bin_start[c * Nz];
-  int64_t p = (int64_t)group_start[c] * NB_GROUP + rank;
+  int c = k / Nz, b0 = c * Nz;
+  if (BATCH) {
+    const NbFrameDev &F = frames[atom_frame[a]];
+    const int col = (k - F.bin0) / F.Nz;
+    c = F.col0 + col;
+    b0 = F.bin0 + col * F.Nz;
+  }
+  const int lo = bin_start[k], hi = bin_start[k + 1];
+  int col_rank = lo - bin_start[b0];
+  for (int j = lo; j < hi; ++j) col_rank += sorted[j] < a ? 1 : 0;
+  int64_t p = (int64_t)group_start[c] * NB_GROUP + col_rank;
   if (p >= places_cap) {
     place_of[a] = -1;
     return;
@@ -645,36 +652,67 @@ __global__ void __launch_bounds__(128) nb_search_t(SearchParams P0, const NbFram
   }
 }
 
-__global__ void nb_unit_count(int64_t groups_cap, const int32_t *__restrict__ sizes,
-                              const int32_t *__restrict__ counts, int64_t list_cap,
-                              int32_t *__restrict__ unit_n) {
-  int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= groups_cap) return;
-  int c = 0;
-  if (g < sizes[NB_SIZE_GROUPS]) c = (int)min((int64_t)counts[g], list_cap);
-  unit_n[g] = (c + NB_UNIT - 1) / NB_UNIT;
+// The units of the lists (64 entries each), in group order: the units of
+// blocks of NB_SCAN_TILE groups, then a pass in which each block adds the
+// units before its own, scans its groups and writes their units.  One block
+// takes the second pass alone.  With a gate (a pruning of the MD step),
+// nothing unless it is set.  `entries` counts the lists' entries.
+__device__ __forceinline__ int nb_group_units(int64_t g, int groups, const int32_t *__restrict__ counts,
+                                              int64_t list_cap) {
+  return g < groups ? ((int)min((int64_t)counts[g], list_cap) + NB_UNIT - 1) / NB_UNIT : 0;
 }
 
-__global__ void nb_unit_write(int64_t groups_cap, const int32_t *__restrict__ unit_n,
-                              const int32_t *__restrict__ unit_start, int64_t units_cap,
-                              int2 *__restrict__ units, int32_t *__restrict__ sizes) {
-  int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (g == 0) {
-    int total = unit_start[groups_cap];
-    sizes[NB_SIZE_UNITS] = total;
-    if (total > units_cap) atomicOr(&sizes[NB_SIZE_OVERFLOW], 4);
+__global__ void __launch_bounds__(NB_SCAN_THREADS) nb_unit_blocks(int64_t groups_cap,
+                                                                  const int32_t *__restrict__ sizes,
+                                                                  const int32_t *__restrict__ counts,
+                                                                  int64_t list_cap, int32_t *__restrict__ block_units,
+                                                                  const int *gate) {
+  __shared__ int sw[32];
+  if (gate && *gate == 0) return;
+  const int groups = (int)min((int64_t)sizes[NB_SIZE_GROUPS], groups_cap);
+  int n = 0;
+#pragma unroll
+  for (int k = 0; k < NB_SCAN_PER_THREAD; ++k)
+    n += nb_group_units((int64_t)blockIdx.x * NB_SCAN_TILE + k * NB_SCAN_THREADS + threadIdx.x, groups, counts,
+                        list_cap);
+  int total;
+  nb_block_exclusive_scan(n, sw, total);
+  if (threadIdx.x == 0) block_units[blockIdx.x] = total;
+}
+
+__global__ void __launch_bounds__(NB_SCAN_THREADS) nb_unit_write(
+    int64_t groups_cap, const int32_t *__restrict__ sizes, const int32_t *__restrict__ counts, int64_t list_cap,
+    const int32_t *__restrict__ block_units, int64_t units_cap, int32_t *__restrict__ unit_start,
+    int2 *__restrict__ units, int32_t *sizes_out, int entries, const int *gate, double *prunes) {
+  __shared__ int sw[32];
+  if (gate && *gate == 0) return;
+  const int groups = (int)min((int64_t)sizes[NB_SIZE_GROUPS], groups_cap);
+  int at = nb_sum_before(block_units, blockIdx.x, sw);
+  int listed = 0;
+  for (int k = 0; k < NB_SCAN_PER_THREAD; ++k) {
+    const int64_t g = (int64_t)blockIdx.x * NB_SCAN_TILE + k * NB_SCAN_THREADS + threadIdx.x;
+    const int n = nb_group_units(g, groups, counts, list_cap);
+    int total;
+    const int first = at + nb_block_exclusive_scan(n, sw, total);
+    at += total;
+    if (g < groups) {
+      unit_start[g] = first;
+      for (int o = 0; o < n; ++o)
+        if (first + o < units_cap) units[first + o] = make_int2((int)g, o);
+      listed += counts[g];
+    }
   }
-  if (g >= groups_cap) return;
-  int s = unit_start[g];
-  for (int k = 0; k < unit_n[g]; ++k)
-    if (s + k < units_cap) units[s + k] = make_int2((int)g, k);
-}
-
-__global__ void nb_count_entries(int64_t groups_cap, const int32_t *sizes,
-                                 const int32_t *__restrict__ counts, int32_t *out) {
-  int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= groups_cap || g >= sizes[NB_SIZE_GROUPS]) return;
-  atomicAdd(&out[NB_SIZE_ENTRIES], counts[g]);
+  if (entries) {
+    int total;
+    nb_block_exclusive_scan(listed, sw, total);
+    if (threadIdx.x == 0 && total > 0) atomicAdd(&sizes_out[NB_SIZE_ENTRIES], total);
+  }
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
+    sizes_out[NB_SIZE_UNITS] = at;
+    if (at > units_cap) atomicOr(&sizes_out[NB_SIZE_OVERFLOW], 4);
+    unit_start[groups] = at;
+    if (prunes) *prunes += 1.0;
+  }
 }
 
 // The pruning of the dual list (MDIR: emitGroupsPrune,
@@ -810,7 +848,7 @@ static int nb_reserve(NbCtx &c, int64_t list_cap, cudaStream_t s) {
   int64_t bins = c.plan_bins + 1;
   if (bins > c.bins_cap) {
     int64_t cap = bins + bins / 4;
-    if (nb_realloc(c.bin_count, cap) || nb_realloc(c.bin_start, cap + 1) || nb_realloc(c.bin_fill, cap))
+    if (nb_realloc(c.bin_count, cap) || nb_realloc(c.bin_start, cap + 1))
       return -1;
     int64_t scr = cap / NB_SCAN_TILE + 8;
     int64_t scr2 = (groups + groups / 4) / NB_SCAN_TILE + 8;
@@ -819,7 +857,7 @@ static int nb_reserve(NbCtx &c, int64_t list_cap, cudaStream_t s) {
   }
   if (cols + 1 > c.cols_cap) {
     int64_t cap = cols + cols / 4 + 1;
-    if (nb_realloc(c.col_groups, cap) || nb_realloc(c.group_start, cap + 1)) return -1;
+    if (nb_realloc(c.group_start, cap + 1)) return -1;
     c.cols_cap = cap;
   }
   bool regroup = groups > c.groups_cap;
@@ -827,7 +865,7 @@ static int nb_reserve(NbCtx &c, int64_t list_cap, cudaStream_t s) {
     int64_t cap = groups + groups / 4 + 16;
     if (nb_realloc(c.order, cap * NB_GROUP) || nb_realloc(c.shift, cap * NB_GROUP) ||
         nb_realloc(c.xw, cap * NB_GROUP) ||
-        nb_realloc(c.group_col, cap) || nb_realloc(c.counts, cap) || nb_realloc(c.counts_lj, cap) || nb_realloc(c.unit_n, cap) ||
+        nb_realloc(c.counts, cap) || nb_realloc(c.counts_lj, cap) ||
         nb_realloc(c.unit_start, cap + 1) || nb_realloc(c.xq, cap * NB_GROUP) ||
         nb_realloc(c.xq_lo, cap * NB_GROUP) ||
         nb_realloc(c.typ_p, cap * NB_GROUP) || nb_realloc(c.acc, cap * NB_GROUP) ||
@@ -900,30 +938,39 @@ static int nb_lj_order(const NbCtx &c) {
 #define NB_SEARCH_FOUR_GROUPS 4000
 static bool nb_search_four(int64_t groups) { return groups < NB_SEARCH_FOUR_GROUPS; }
 
-// Launches one build on `s`. Returns 0; the sizes are left in c.sizes (device).
+// The units of the lists `counts` into `units` (nb_unit_write).
+static void nb_units_run(NbCtx &c, const int32_t *counts, int32_t *unit_start, int2 *units, int32_t *sizes_out,
+                         int entries, const int *gate, double *prunes, cudaStream_t s) {
+  const int blocks = blocks_for(c.groups_cap, NB_SCAN_TILE);
+  if (blocks > 1)
+    nb_unit_blocks<<<blocks, NB_SCAN_THREADS, 0, s>>>(c.groups_cap, c.sizes, counts, c.list_cap, c.scan_scratch, gate);
+  nb_unit_write<<<blocks, NB_SCAN_THREADS, 0, s>>>(c.groups_cap, c.sizes, counts, c.list_cap, c.scan_scratch,
+                                                   c.units_cap, unit_start, units, sizes_out, entries, gate, prunes);
+}
+
+// Launches one build on `s`; the sizes are left in c.sizes (device).  The
+// chain is nine launches and two memsets (keys, scan, scatter, columns, places,
+// search, units), two fewer where a block takes a scan alone: the small
+// kernels of a build are each a launch's latency, and 24 of them took as
+// long as the search for 900 atoms.
 static void nb_build_launch(NbCtx &c, const double *x, const double box[3], cudaStream_t s) {
   const NbGrid &G = c.grid;
   int64_t n = c.n;
   int nbins = G.nbins();
-  cudaMemsetAsync(c.sizes, 0, sizeof(int32_t) * NB_SIZE_COUNT, s);
   cudaMemsetAsync(c.bin_count, 0, sizeof(int32_t) * (nbins + 1), s);
-  cudaMemsetAsync(c.bin_fill, 0, sizeof(int32_t) * (nbins + 1), s);
   cudaMemsetAsync(c.order, 0xff, sizeof(int32_t) * c.places_cap, s);
   nb_keys<<<blocks_for(n, 256), 256, 0, s>>>(n, x, box[0], box[1], box[2], c.tilt[0], c.tilt[1], c.tilt[2],
                                             G.Nx, G.Ny, G.Nz,
-                                            1.0f / G.wx, 1.0f / G.wy, 1.0f / G.hz, c.key,
-                                            c.bin_count, c.atom_xw, c.atom_shift, c.sizes);
+                                            1.0f / G.wx, 1.0f / G.wy, 1.0f / G.hz, c.key, c.rank,
+                                            c.bin_count, c.atom_xw, c.atom_shift);
   nb_scan(c.bin_count, c.bin_start, nbins + 1, nullptr, c.scan_scratch, s);
-  nb_scatter<<<blocks_for(n, 256), 256, 0, s>>>(n, c.key, c.bin_start, c.bin_fill, c.sorted);
-  nb_bin_sort<<<blocks_for(nbins + 1, 256), 256, 0, s>>>(nbins + 1, c.bin_start, c.sorted);
-  nb_col_groups<<<blocks_for(G.ncol(), 256), 256, 0, s>>>(G.ncol(), G.Nz, c.bin_start, c.col_groups);
-  nb_scan(c.col_groups, c.group_start, G.ncol(), nullptr, c.scan_scratch, s);
-  nb_group_cols<<<blocks_for(G.ncol(), 256), 256, 0, s>>>(G.ncol(), c.group_start, c.groups_cap,
-                                                         c.group_col, c.sizes);
-  nb_places<<<blocks_for(n, 256), 256, 0, s>>>((int)n, c.bin_start, nbins, c.sorted, c.key, G.Nz,
-                                              c.group_start, c.places_cap, c.atom_xw, c.atom_shift, c.type,
-                                              nb_lj_order(c) == 1 ? c.lj_on : nullptr, c.order, c.place_of, c.shift,
-                                              c.xw);
+  nb_scatter<<<blocks_for(n, 256), 256, 0, s>>>(n, c.key, c.rank, c.bin_start, c.sorted);
+  nb_columns<false><<<1, 1024, 0, s>>>(G.ncol(), G.Nz, nbins, c.bin_start, nullptr, nullptr, c.groups_cap,
+                                       c.group_start, c.sizes);
+  nb_places<false><<<blocks_for(n, 256), 256, 0, s>>>((int)n, c.bin_start, nbins, c.sorted, c.key, G.Nz, nullptr,
+                                                     nullptr, c.group_start, c.places_cap, c.atom_xw, c.atom_shift,
+                                                     c.type, nb_lj_order(c) == 1 ? c.lj_on : nullptr, c.order,
+                                                     c.place_of, c.shift, c.xw);
   SearchParams P;
   P.Lx = (float)box[0];
   P.Ly = (float)box[1];
@@ -951,13 +998,7 @@ static void nb_build_launch(NbCtx &c, const double *x, const double box[3], cuda
                                 : (four ? nb_search_t<4, false> : nb_search_t<1, false>);
   kernel<<<blocks, 128, 0, s>>>(P, nullptr, nullptr, c.sizes, c.order, c.xw, c.group_start, c.bin_start, c.excl_off,
                                 c.excl, c.slab, c.counts, c.counts_lj, c.sizes);
-  nb_unit_count<<<blocks_for(c.groups_cap, 256), 256, 0, s>>>(c.groups_cap, c.sizes, c.counts,
-                                                             c.list_cap, c.unit_n);
-  nb_scan(c.unit_n, c.unit_start, (int)c.groups_cap, nullptr, c.scan_scratch, s);
-  nb_unit_write<<<blocks_for(c.groups_cap, 256), 256, 0, s>>>(c.groups_cap, c.unit_n, c.unit_start,
-                                                             c.units_cap, c.units, c.sizes);
-  nb_count_entries<<<blocks_for(c.groups_cap, 256), 256, 0, s>>>(c.groups_cap, c.sizes, c.counts,
-                                                                c.sizes);
+  nb_units_run(c, c.counts, c.unit_start, c.units, c.sizes, 1, nullptr, nullptr, s);
 }
 
 void nb_build_launch_public(NbCtx &c, const double *x, const double box[3], cudaStream_t s) {
@@ -968,7 +1009,7 @@ int nb_reserve_inner(NbCtx &c, cudaStream_t s) {
   // the inner buffers follow the outer capacities
   int64_t G = c.groups_cap, C = c.list_cap, U = c.units_cap;
   c.slab_in_entries = 0;
-  if (nb_realloc(c.slab_in, G * C) || nb_realloc(c.counts_in, G) || nb_realloc(c.unit_n_in, G) ||
+  if (nb_realloc(c.slab_in, G * C) || nb_realloc(c.counts_in, G) ||
       nb_realloc(c.unit_start_in, G + 1) || nb_realloc(c.units_in, U))
     return -1;
   c.slab_in_entries = G * C;
@@ -995,55 +1036,8 @@ void nb_prune_run(NbCtx &c, const double box[3], cudaStream_t s) {
                                                         c.counts, c.order, c.xq, c.slab_in, c.counts_in, nullptr,
                                                         nullptr, nullptr);
   }
-  nb_unit_count<<<blocks_for(c.groups_cap, 256), 256, 0, s>>>(c.groups_cap, c.sizes, c.counts_in, c.list_cap,
-                                                             c.unit_n_in);
-  nb_scan(c.unit_n_in, c.unit_start_in, (int)c.groups_cap, nullptr, c.scan_scratch, s);
-  nb_unit_write<<<blocks_for(c.groups_cap, 256), 256, 0, s>>>(c.groups_cap, c.unit_n_in, c.unit_start_in,
-                                                             c.units_cap, c.units_in, c.sizes_in);
+  nb_units_run(c, c.counts_in, c.unit_start_in, c.units_in, c.sizes_in, 0, nullptr, nullptr, s);
 }
-
-namespace {
-
-// The units of the lists in one block: a scan of the groups' unit counts,
-// then the units (group, ordinal) in group order, the same as the
-// three-kernel path; with a gate, nothing unless it is set.  Counts one
-// more pruning in *prunes.
-__global__ void __launch_bounds__(1024) nb_units_one_block(int64_t groups_cap, const int32_t *__restrict__ sizes,
-                                                           const int32_t *__restrict__ counts, int64_t list_cap,
-                                                           int64_t units_cap, int32_t *__restrict__ unit_start,
-                                                           int2 *__restrict__ units, int32_t *__restrict__ sizes_out,
-                                                           const int *gate, double *prunes) {
-  __shared__ int s_part[1024];
-  if (gate && *gate == 0) return;
-  int G = (int)min((int64_t)sizes[NB_SIZE_GROUPS], groups_cap);
-  int t = threadIdx.x;
-  int per = (G + (int)blockDim.x - 1) / (int)blockDim.x;
-  int g0 = min(G, t * per), g1 = min(G, g0 + per);
-  int local = 0;
-  for (int g = g0; g < g1; ++g) local += ((int)min((int64_t)counts[g], list_cap) + NB_UNIT - 1) / NB_UNIT;
-  s_part[t] = local;
-  __syncthreads();
-  for (int o = 1; o < (int)blockDim.x; o <<= 1) {
-    int y = t >= o ? s_part[t - o] : 0;
-    __syncthreads();
-    s_part[t] += y;
-    __syncthreads();
-  }
-  int at = s_part[t] - local;
-  for (int g = g0; g < g1; ++g) {
-    int n = ((int)min((int64_t)counts[g], list_cap) + NB_UNIT - 1) / NB_UNIT;
-    unit_start[g] = at;
-    for (int k = 0; k < n; ++k)
-      if (at + k < units_cap) units[at + k] = make_int2(g, k);
-    at += n;
-  }
-  if (t == (int)blockDim.x - 1) {
-    sizes_out[NB_SIZE_UNITS] = s_part[t];
-    if (prunes) *prunes += 1.0;
-  }
-}
-
-}  // namespace
 
 void nb_prune_gated(NbCtx &c, const double box[3], const int *gate, const double *x, double *x_prune,
                     double *prunes, int32_t *unit_counter, cudaStream_t s) {
@@ -1067,8 +1061,7 @@ void nb_prune_gated(NbCtx &c, const double box[3], const int *gate, const double
                                                         c.counts, c.order, c.xq, c.slab_in, c.counts_in, gate, x,
                                                         x_prune);
   }
-  nb_units_one_block<<<1, 1024, 0, s>>>(c.groups_cap, c.sizes, c.counts_in, c.list_cap, c.units_cap, c.unit_start_in,
-                                       c.units_in, c.sizes_in, gate, prunes);
+  nb_units_run(c, c.counts_in, c.unit_start_in, c.units_in, c.sizes_in, 0, gate, prunes, s);
 }
 
 // One complete build with count-then-grow: the list capacity C grows to a
@@ -1084,7 +1077,7 @@ int nb_build_run(NbCtx &c, const double *x, const double box[3], cudaStream_t s)
   c.plan_bins = G.nbins();
   if (!c.key) {
     if (nb_realloc(c.key, c.n) || nb_realloc(c.sorted, c.n) || nb_realloc(c.atom_xw, c.n) ||
-        nb_realloc(c.atom_shift, c.n) || nb_realloc(c.place_of, c.n))
+        nb_realloc(c.atom_shift, c.n) || nb_realloc(c.place_of, c.n) || nb_realloc(c.rank, c.n))
       return -1;
   }
   for (int attempt = 0; attempt < 8; ++attempt) {
@@ -1206,9 +1199,8 @@ namespace {
 
 __global__ void nb_batch_keys(int64_t n, const double *__restrict__ x, const int32_t *__restrict__ atom_frame,
                               const NbFrameDev *__restrict__ frames, int nbins, int32_t *__restrict__ key,
-                              int32_t *__restrict__ atom_col, int32_t *__restrict__ bin_count,
-                              float4 *__restrict__ atom_xw, char4 *__restrict__ atom_shift,
-                              int32_t *__restrict__ sizes) {
+                              int32_t *__restrict__ rank, int32_t *__restrict__ bin_count,
+                              float4 *__restrict__ atom_xw, char4 *__restrict__ atom_shift) {
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const NbFrameDev &F = frames[atom_frame[i]];
@@ -1223,9 +1215,7 @@ __global__ void nb_batch_keys(int64_t n, const double *__restrict__ x, const int
   }
   if (!ok) {
     key[i] = nbins;
-    atom_col[i] = -1;
-    atomicAdd(&bin_count[nbins], 1);
-    atomicAdd(&sizes[NB_SIZE_NAN], 1);
+    rank[i] = atomicAdd(&bin_count[nbins], 1);
     atom_xw[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     atom_shift[i] = make_char4(0, 0, 0, 0);
     return;
@@ -1237,64 +1227,23 @@ __global__ void nb_batch_keys(int64_t n, const double *__restrict__ x, const int
   int col = ky * F.Nx + kx;
   int k = F.bin0 + col * F.Nz + kz;
   key[i] = k;
-  atom_col[i] = F.col0 + col;
-  atomicAdd(&bin_count[k], 1);
+  rank[i] = atomicAdd(&bin_count[k], 1);
   atom_xw[i] = make_float4(w0, w1, w2, 1.f);
   atom_shift[i] = make_char4((signed char)S0, (signed char)S1, (signed char)S2, 0);
 }
 
-__global__ void nb_batch_col_groups(int ncol, const int32_t *__restrict__ col_frame,
-                                    const NbFrameDev *__restrict__ frames, const int32_t *__restrict__ bin_start,
-                                    int32_t *__restrict__ col_groups) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
+// Each group's frame and its frame's cell, a thread a column.
+__global__ void nb_batch_group_frames(int ncol, const int32_t *__restrict__ group_start, int64_t groups_cap,
+                                      const int32_t *__restrict__ col_frame, const NbFrameDev *__restrict__ frames,
+                                      int32_t *__restrict__ group_frame, float4 *__restrict__ group_L) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= ncol) return;
-  const NbFrameDev &F = frames[col_frame[c]];
-  int b0 = F.bin0 + (c - F.col0) * F.Nz;
-  int nc = bin_start[b0 + F.Nz] - bin_start[b0];
-  col_groups[c] = (nc + NB_GROUP - 1) / NB_GROUP;
-}
-
-__global__ void nb_batch_places(int nsorted_max, const int32_t *__restrict__ bin_start, int nvalid_bins,
-                                const int32_t *__restrict__ sorted, const int32_t *__restrict__ atom_col,
-                                const int32_t *__restrict__ col_frame, const NbFrameDev *__restrict__ frames,
-                                const int32_t *__restrict__ group_start, int64_t places_cap,
-                                const float4 *__restrict__ atom_xw, const char4 *__restrict__ atom_shift,
-                                const int32_t *__restrict__ type, const int32_t *__restrict__ lj_on,
-                                int32_t *__restrict__ order, int32_t *__restrict__ place_of,
-                                char4 *__restrict__ shift, float4 *__restrict__ xw) {
-  int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= nsorted_max) return;
-  int nvalid = bin_start[nvalid_bins];
-  int a = sorted[s];
-  if (s >= nvalid) {
-    place_of[a] = -1;
-    return;
+  const int f = col_frame[c];
+  const float4 L = make_float4(frames[f].Lf0, frames[f].Lf1, frames[f].Lf2, 0.f);
+  for (int g = group_start[c]; g < group_start[c + 1] && g < groups_cap; ++g) {
+    group_frame[g] = f;
+    group_L[g] = L;
   }
-  int c = atom_col[a];
-  const NbFrameDev &F = frames[col_frame[c]];
-  int rank = s - bin_start[F.bin0 + (c - F.col0) * F.Nz];
-  int64_t p = (int64_t)group_start[c] * NB_GROUP + rank;
-  if (p >= places_cap) {
-    place_of[a] = -1;
-    return;
-  }
-  order[p] = a;
-  place_of[a] = (int32_t)p;
-  shift[p] = atom_shift[a];
-  float4 v = atom_xw[a];
-  v.w = __int_as_float(a | (lj_on && lj_on[type[a]] != 0 ? NB_ATOM_LJ : 0));
-  xw[p] = v;
-}
-
-__global__ void nb_batch_group_frames(int64_t groups_cap, const int32_t *__restrict__ sizes,
-                                      const int32_t *__restrict__ group_col, const int32_t *__restrict__ col_frame,
-                                      const NbFrameDev *__restrict__ frames, int32_t *__restrict__ group_frame,
-                                      float4 *__restrict__ group_L) {
-  int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= groups_cap || g >= sizes[NB_SIZE_GROUPS]) return;
-  int f = col_frame[group_col[g]];
-  group_frame[g] = f;
-  group_L[g] = make_float4(frames[f].Lf0, frames[f].Lf1, frames[f].Lf2, 0.f);
 }
 
 // The units of frame f: [frame_units[2f], frame_units[2f + 1]).
@@ -1370,27 +1319,20 @@ static void nb_batch_build_launch(mdrtNbBatch &b, const double *x, cudaStream_t 
   int64_t n = c.n;
   int nbins = (int)c.plan_bins;
   int ncol = (int)c.plan_cols;
-  cudaMemsetAsync(c.sizes, 0, sizeof(int32_t) * NB_SIZE_COUNT, s);
   cudaMemsetAsync(c.bin_count, 0, sizeof(int32_t) * (nbins + 1), s);
-  cudaMemsetAsync(c.bin_fill, 0, sizeof(int32_t) * (nbins + 1), s);
   cudaMemsetAsync(c.order, 0xff, sizeof(int32_t) * c.places_cap, s);
-  nb_batch_keys<<<blocks_for(n, 256), 256, 0, s>>>(n, x, b.atom_frame, b.frames_dev, nbins, c.key, b.atom_col,
-                                                  c.bin_count, c.atom_xw, c.atom_shift, c.sizes);
+  nb_batch_keys<<<blocks_for(n, 256), 256, 0, s>>>(n, x, b.atom_frame, b.frames_dev, nbins, c.key, c.rank,
+                                                  c.bin_count, c.atom_xw, c.atom_shift);
   nb_scan(c.bin_count, c.bin_start, nbins + 1, nullptr, c.scan_scratch, s);
-  nb_scatter<<<blocks_for(n, 256), 256, 0, s>>>(n, c.key, c.bin_start, c.bin_fill, c.sorted);
-  nb_bin_sort<<<blocks_for(nbins + 1, 256), 256, 0, s>>>(nbins + 1, c.bin_start, c.sorted);
-  nb_batch_col_groups<<<blocks_for(ncol, 256), 256, 0, s>>>(ncol, b.col_frame, b.frames_dev, c.bin_start,
-                                                           c.col_groups);
-  nb_scan(c.col_groups, c.group_start, ncol, nullptr, c.scan_scratch, s);
-  nb_group_cols<<<blocks_for(ncol, 256), 256, 0, s>>>(ncol, c.group_start, c.groups_cap, c.group_col, c.sizes);
-  nb_batch_places<<<blocks_for(n, 256), 256, 0, s>>>((int)n, c.bin_start, nbins, c.sorted, b.atom_col,
-                                                    b.col_frame, b.frames_dev, c.group_start, c.places_cap,
-                                                    c.atom_xw, c.atom_shift, c.type,
-                                                    nb_lj_order(c) == 1 ? c.lj_on : nullptr, c.order, c.place_of,
-                                                    c.shift, c.xw);
-  nb_batch_group_frames<<<blocks_for(c.groups_cap, 256), 256, 0, s>>>(c.groups_cap, c.sizes, c.group_col,
-                                                                     b.col_frame, b.frames_dev, b.group_frame,
-                                                                     b.group_L);
+  nb_scatter<<<blocks_for(n, 256), 256, 0, s>>>(n, c.key, c.rank, c.bin_start, c.sorted);
+  nb_columns<true><<<1, 1024, 0, s>>>(ncol, 1, nbins, c.bin_start, b.frames_dev, b.col_frame, c.groups_cap,
+                                      c.group_start, c.sizes);
+  nb_batch_group_frames<<<blocks_for(ncol, 128), 128, 0, s>>>(ncol, c.group_start, c.groups_cap, b.col_frame,
+                                                             b.frames_dev, b.group_frame, b.group_L);
+  nb_places<true><<<blocks_for(n, 256), 256, 0, s>>>((int)n, c.bin_start, nbins, c.sorted, c.key, 1, b.frames_dev,
+                                                    b.atom_frame, c.group_start, c.places_cap, c.atom_xw,
+                                                    c.atom_shift, c.type, nb_lj_order(c) == 1 ? c.lj_on : nullptr,
+                                                    c.order, c.place_of, c.shift, c.xw);
   SearchParams P = {};
   P.groups_cap = c.groups_cap;
   P.list_cap = c.list_cap;
@@ -1400,12 +1342,7 @@ static void nb_batch_build_launch(mdrtNbBatch &b, const double *x, cudaStream_t 
   auto kernel = four ? nb_search_t<4, true> : nb_search_t<1, true>;
   kernel<<<blocks, 128, 0, s>>>(P, b.frames_dev, b.group_frame, c.sizes, c.order, c.xw, c.group_start, c.bin_start,
                                 c.excl_off, c.excl, c.slab, c.counts, c.counts_lj, c.sizes);
-  nb_unit_count<<<blocks_for(c.groups_cap, 256), 256, 0, s>>>(c.groups_cap, c.sizes, c.counts, c.list_cap,
-                                                             c.unit_n);
-  nb_scan(c.unit_n, c.unit_start, (int)c.groups_cap, nullptr, c.scan_scratch, s);
-  nb_unit_write<<<blocks_for(c.groups_cap, 256), 256, 0, s>>>(c.groups_cap, c.unit_n, c.unit_start, c.units_cap,
-                                                             c.units, c.sizes);
-  nb_count_entries<<<blocks_for(c.groups_cap, 256), 256, 0, s>>>(c.groups_cap, c.sizes, c.counts, c.sizes);
+  nb_units_run(c, c.counts, c.unit_start, c.units, c.sizes, 1, nullptr, nullptr, s);
   nb_batch_frame_units<<<blocks_for(b.frames, 128), 128, 0, s>>>(b.frames, b.frames_dev, c.group_start,
                                                                 c.unit_start, b.frame_units);
 }
@@ -1417,7 +1354,7 @@ int nb_batch_build_run(mdrtNbBatch &b, const double *x, cudaStream_t s) {
   int64_t cap = std::max<int64_t>(c.list_cap, hint);
   if (!c.key) {
     if (nb_realloc(c.key, c.n) || nb_realloc(c.sorted, c.n) || nb_realloc(c.atom_xw, c.n) ||
-        nb_realloc(c.atom_shift, c.n) || nb_realloc(c.place_of, c.n) || nb_realloc(b.atom_col, c.n))
+        nb_realloc(c.atom_shift, c.n) || nb_realloc(c.place_of, c.n) || nb_realloc(c.rank, c.n))
       return -1;
   }
   if (!b.frame_units && nb_realloc(b.frame_units, 2 * (int64_t)b.frames)) return -1;

@@ -88,17 +88,16 @@ struct NbCtx {
   char4 *shift = nullptr;  // per place
   float4 *xw = nullptr;    // per place, f32 wrapped at the build, the atom's number in w
   int32_t *group_start = nullptr;  // per column + 1
-  int32_t *group_col = nullptr;    // per group
   int2 *slab = nullptr;            // groups_cap * list_cap entries
   int32_t *counts = nullptr;       // per group
-  int32_t *unit_n = nullptr, *unit_start = nullptr;  // per group (+1)
+  int32_t *unit_start = nullptr;  // per group (+1)
   int2 *units = nullptr;           // (group, ordinal)
   int32_t *sizes = nullptr;        // NB_SIZE_COUNT ints on the device
   int32_t *h_sizes = nullptr;      // pinned mirror
   int32_t *status = nullptr;       // device status word
   // build scratch
-  int32_t *key = nullptr, *bin_count = nullptr, *bin_start = nullptr, *bin_fill = nullptr;
-  int32_t *sorted = nullptr, *col_groups = nullptr, *scan_scratch = nullptr;
+  int32_t *key = nullptr, *rank = nullptr, *bin_count = nullptr, *bin_start = nullptr;
+  int32_t *sorted = nullptr, *scan_scratch = nullptr;
   float4 *atom_xw = nullptr;
   char4 *atom_shift = nullptr;
   // per-step frames and accumulators (place order)
@@ -123,7 +122,7 @@ struct NbCtx {
   int2 *slab_in = nullptr;
   int64_t slab_in_entries = 0;  // the allocation of slab_in
   int32_t *counts_in = nullptr;
-  int32_t *unit_n_in = nullptr, *unit_start_in = nullptr;
+  int32_t *unit_start_in = nullptr;
   int2 *units_in = nullptr;
   int32_t *sizes_in = nullptr;  // NB_SIZE_UNITS of the inner list (device)
   int64_t prunes = 0;
@@ -229,7 +228,6 @@ struct mdrtNbBatch {
   std::vector<NbFrameDev> h_frames;
   NbFrameDev *frames_dev = nullptr;
   int32_t *atom_frame = nullptr;  // per atom
-  int32_t *atom_col = nullptr;    // per atom: its column at the build
   int32_t *col_frame = nullptr;   // per column
   int32_t *group_frame = nullptr; // per group
   float4 *group_L = nullptr;      // per group: the frame's cell
