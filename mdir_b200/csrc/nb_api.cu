@@ -220,6 +220,9 @@ int32_t mdrtNbDestroy(mdrtNb *ctx) {
     if (g.exec) cudaGraphExecDestroy(g.exec);
   ctx->graphs.clear();
   if (ctx->capture) cudaStreamDestroy(ctx->capture);
+  if (ctx->side) cudaStreamDestroy(ctx->side);
+  if (ctx->ev_fork) cudaEventDestroy(ctx->ev_fork);
+  if (ctx->ev_join) cudaEventDestroy(ctx->ev_join);
   nb_pme_release(c);
   nb_free(c.q); nb_free(c.type); nb_free(c.lj); nb_free(c.ljf); nb_free(c.sigeps);
   nb_free(c.lj_on); nb_free(c.counts_lj);
@@ -502,6 +505,13 @@ static int32_t nb_build_entry(mdrtNb *ctx, const double *x, int64_t n, const dou
   cudaStream_t st = (cudaStream_t)stream;
   if (nb_build_run(c, x, box, st)) return MDRT_NB_CUDA_ERROR;
   for (int k = 0; k < 3; ++k) c.tilt_built[k] = c.tilt[k];
+  if (!ctx->side) {
+    int least = 0, greatest = 0;
+    CK(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+    CK(cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming));
+    CK(cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming));
+    CK(cudaStreamCreateWithPriority(&ctx->side, cudaStreamNonBlocking, greatest));
+  }
   if (!c.x_build) CK(cudaMalloc(&c.x_build, sizeof(double) * 3 * c.n));
   CK(cudaMemcpyAsync(c.x_build, x, sizeof(double) * 3 * c.n, cudaMemcpyDeviceToDevice, st));
   if (sizes_out)
@@ -511,13 +521,13 @@ static int32_t nb_build_entry(mdrtNb *ctx, const double *x, int64_t n, const dou
 }
 
 static int32_t nb_force_entry(mdrtNb *ctx, const double *x, const double box[3], uint32_t flags, double *forces,
-                              void *stream);
+                              void *stream, bool beside);
 
 int32_t mdrtNbForce(mdrtNb *ctx, const double *x, const double box[3], uint32_t flags, double *forces,
                     void *stream) {
   if (!ctx || !x || !forces) return MDRT_NB_INVALID_ARGUMENT;
   if (nb_triclinic(ctx->c)) return MDRT_NB_INVALID_BOX;  // built in a triclinic cell
-  return nb_force_entry(ctx, x, box, flags, forces, stream);
+  return nb_force_entry(ctx, x, box, flags, forces, stream, true);
 }
 
 int32_t mdrtNbForceTriclinic(mdrtNb *ctx, const double *x, const double cell[6], uint32_t flags, double *forces,
@@ -527,11 +537,21 @@ int32_t mdrtNbForceTriclinic(mdrtNb *ctx, const double *x, const double cell[6],
   if (s) return s;
   for (int k = 0; k < 3; ++k)
     if (cell[3 + k] != ctx->c.tilt_built[k]) return MDRT_NB_INVALID_BOX;  // a cell change needs a build
-  return nb_force_entry(ctx, x, cell, flags, forces, stream);
+  return nb_force_entry(ctx, x, cell, flags, forces, stream, true);
 }
 
+// Atoms from which a force call's reciprocal chain runs beside its pairs: the
+// fork and join cost the host about 4 µs a call, which a small system, bound
+// by its launches, does not get back (3,000 atoms: 39 µs a call with one
+// stream, 43 with two; 8,013: 61 and 51; 23,550: 64 and 54).  With energies the
+// pairs' branch is longer (their sums): 3,000 atoms 64 and 52 µs.
+#define NB_BESIDE_ATOMS 6000
+#define NB_BESIDE_ENERGY_ATOMS 2000
+
+// `beside`: the reciprocal chain on the context's own stream beside the
+// pairs (the frames entries keep one stream a lane: their lanes fill the GPU).
 static int32_t nb_force_entry(mdrtNb *ctx, const double *x, const double box[3], uint32_t flags, double *forces,
-                              void *stream) {
+                              void *stream, bool beside) {
   NbCtx &c = ctx->c;
   if (!c.built) return MDRT_NB_NOT_BUILT;
   int s = check_box(c, box);
@@ -543,9 +563,21 @@ static int32_t nb_force_entry(mdrtNb *ctx, const double *x, const double box[3],
   bool pairs = !(flags & MDRT_NB_NO_PAIRS);
   bool excluded = !(flags & MDRT_NB_NO_EXCLUDED);
   bool pme = c.pme.on && !(flags & MDRT_NB_NO_PME) && c.beta > 0.0;
-  if (!(flags & MDRT_NB_ACCUMULATE)) CK(cudaMemsetAsync(forces, 0, sizeof(double) * 3 * c.n, st));
   if (energy) CK(cudaMemsetAsync(c.energy, 0, sizeof(double) * NB_E_SLOTS, st));
   nb_gather_frames(c, x, box, st);
+  const bool gathers = pme && nb_finish_gathers(c);
+  const bool potential = (flags & MDRT_NB_POTENTIAL) != 0;
+  beside = beside && pme && pairs && ctx->side && c.n >= (energy ? NB_BESIDE_ENERGY_ATOMS : NB_BESIDE_ATOMS);
+  if (beside) {
+    CK(cudaEventRecord(ctx->ev_fork, st));
+    CK(cudaStreamWaitEvent(ctx->side, ctx->ev_fork, 0));
+    const int rc = nb_pme_run(c, box, energy, potential, ctx->side, !gathers);
+    CK(cudaEventRecord(ctx->ev_join, ctx->side));  // joined below, also after an error
+    if (rc) {
+      CK(cudaStreamWaitEvent(st, ctx->ev_join, 0));
+      return MDRT_NB_CUDA_ERROR;
+    }
+  }
   bool pairs_done = false;
   if ((flags & MDRT_NB_PRUNE) && c.inner_reach > 0.0) {
     // the pruning at x, and, for forces outside the deterministic mode, the
@@ -568,13 +600,20 @@ static int32_t nb_force_entry(mdrtNb *ctx, const double *x, const double box[3],
   if (pairs && !pairs_done) nb_pairs_run(c, box, energy, st);
   if (excluded) nb_excluded_run(c, box, energy, st);
   if (energy && (pairs || excluded)) nb_reduce_energy(c, pairs, excluded, st);
-  if (pme) {
-    if (nb_pme_run(c, box, energy, (flags & MDRT_NB_POTENTIAL) != 0, st)) return MDRT_NB_CUDA_ERROR;
+  if (beside) {
+    CK(cudaStreamWaitEvent(st, ctx->ev_join, 0));
+  } else if (pme) {
+    if (nb_pme_run(c, box, energy, potential, st, !gathers)) return MDRT_NB_CUDA_ERROR;
   }
-  bool keep_pme = c.pme.on;
-  if (!pme) c.pme.on = false;  // finish without the PME forces of a skipped sum
-  nb_finish_forces(c, forces, 1, st);
-  c.pme.on = keep_pme;
+  const int accumulate = flags & MDRT_NB_ACCUMULATE ? 1 : 0;
+  if (gathers) {
+    nb_finish_gather_run(c, box, forces, accumulate, potential, st);
+  } else {
+    bool keep_pme = c.pme.on;
+    if (!pme) c.pme.on = false;  // finish without the PME forces of a skipped sum
+    nb_finish_forces(c, forces, accumulate, st);
+    c.pme.on = keep_pme;
+  }
   CK(cudaGetLastError());
   return MDRT_NB_OK;
 }
@@ -612,7 +651,7 @@ int32_t mdrtNbForceFrames(mdrtNb *ctx, const double *x, int64_t x_stride, int64_
   if (!box) return MDRT_NB_INVALID_ARGUMENT;
   auto run = [&](cudaStream_t s) -> int32_t {
     for (int64_t k = 0; k < count; ++k) {
-      int32_t r = nb_force_entry(ctx, x + k * x_stride, box, flags, forces + k * f_stride, s);
+      int32_t r = nb_force_entry(ctx, x + k * x_stride, box, flags, forces + k * f_stride, s, false);
       if (r) return r;
       if (potentials && nb_pme_potential_grid(ctx->c, potentials + k * p_stride, s)) return MDRT_NB_CUDA_ERROR;
     }

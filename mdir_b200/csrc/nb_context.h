@@ -21,7 +21,8 @@ struct NbPme {
   int order = 4;
   bool on = false;
   cufftHandle fwd = 0, bwd = 0;
-  float *grid = nullptr;        // K0*K1*K2 real grid
+  float *grid = nullptr;        // K0*K1*K2 charge grid, empty between evaluations
+  float *phi = nullptr;         // the potential of the last evaluation on the same grid
   float2 *spec = nullptr;       // K0*K1*(K2/2+1)
   unsigned long long *fixed = nullptr;  // deterministic spreading, K0*K1*K2
   float *moduli = nullptr;      // |b|^2 tables: K0 + K1 + K2 floats
@@ -189,6 +190,9 @@ struct mdrtNb {
   NbCtx c;
   std::vector<NbFrameGraph> graphs;
   uint64_t graph_clock = 0;
+  // the reciprocal chain of a force call runs on `side` beside its pairs
+  cudaStream_t side = nullptr;
+  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   cudaStream_t capture = nullptr;  // the frames graphs are captured on this stream
   int64_t graph_captures = 0, graph_replays = 0;
   // a started displacement test (mdrtNbDisplacementStart): the event after
@@ -331,7 +335,14 @@ void nb_finish_forces(NbCtx &c, double *forces, int accumulate, cudaStream_t s);
 void nb_reduce_energy(NbCtx &c, bool pairs, bool excluded, cudaStream_t s);
 int nb_pme_setup(NbCtx &c, int k0, int k1, int k2, int order);
 void nb_pme_release(NbCtx &c);
-int nb_pme_run(NbCtx &c, const double box[3], bool energy, bool potential, cudaStream_t s);
+// With `gather`, the forces (and, when asked, the potentials) of the places
+// as well; else the potential grid alone, for nb_finish_gather_run.
+int nb_pme_run(NbCtx &c, const double box[3], bool energy, bool potential, cudaStream_t s, bool gather = true);
+// Whether the finish can gather the PME forces itself (orders 4 and 8), and
+// that finish: the places' forces with the reciprocal ones from the grid.
+bool nb_finish_gathers(const NbCtx &c);
+void nb_finish_gather_run(NbCtx &c, const double box[3], double *forces, int accumulate, bool potential,
+                          cudaStream_t s);
 // The parameter gradient (mdrtNbParameterGradient) summed over `count`
 // frames (x + k x_stride; cotangent + k c_stride; phi + k p_stride when phi
 // is given).  mode 0: the product sum_k g_k . dF_k/dtheta for the cotangent

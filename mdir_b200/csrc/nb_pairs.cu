@@ -743,11 +743,14 @@ __global__ void nb_batch_sums(int nframes, const int32_t *__restrict__ frame_uni
 // of the pairs, the excluded pairs and PME; the accumulators are cleared
 // for the next evaluation.
 template <bool FIXED>
-__global__ void nb_finish(int64_t places, const int32_t *__restrict__ sizes,
-                          const int32_t *__restrict__ order, float4 *__restrict__ acc,
+__global__ void nb_finish(int64_t places, int64_t n, const int32_t *__restrict__ sizes,
+                          const int32_t *__restrict__ order, const int32_t *__restrict__ place_of, float4 *__restrict__ acc,
                           unsigned long long *__restrict__ accf, const float4 *__restrict__ pme_force,
                           double *__restrict__ forces, int accumulate) {
   int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  // an atom with no place (not finite at the build) gets zeros
+  if (!accumulate && p < n && sizes[NB_SIZE_NAN] > 0 && place_of[p] < 0)
+    forces[3 * p] = forces[3 * p + 1] = forces[3 * p + 2] = 0.0;
   if (p >= places || p >= sizes[NB_SIZE_PLACES]) return;
   int a = order[p];
   double f0, f1, f2;
@@ -1242,10 +1245,10 @@ void nb_excluded_run(NbCtx &c, const double box[3], bool energy, cudaStream_t s)
 void nb_finish_forces(NbCtx &c, double *forces, int accumulate, cudaStream_t s) {
   const float4 *pf = c.pme.on ? (const float4 *)c.pme.pme_force : nullptr;
   if (c.deterministic)
-    nb_finish<true><<<blocks_for(c.places_cap, 256), 256, 0, s>>>(c.places_cap, c.sizes, c.order, c.acc,
+    nb_finish<true><<<blocks_for(c.places_cap, 256), 256, 0, s>>>(c.places_cap, c.n, c.sizes, c.order, c.place_of, c.acc,
                                                                  c.acc_fixed, pf, forces, accumulate);
   else
-    nb_finish<false><<<blocks_for(c.places_cap, 256), 256, 0, s>>>(c.places_cap, c.sizes, c.order, c.acc,
+    nb_finish<false><<<blocks_for(c.places_cap, 256), 256, 0, s>>>(c.places_cap, c.n, c.sizes, c.order, c.place_of, c.acc,
                                                                   c.acc_fixed, pf, forces, accumulate);
 }
 

@@ -775,6 +775,90 @@ __global__ void __launch_bounds__(128) nb_pme_gather_split(GridParams G, int64_t
   if (pot) pot[p] = e;
 }
 
+// The finish of a force call that gathers the reciprocal forces itself: P
+// threads a place (as nb_pme_gather_split), whose first three write one
+// component each of the atom's force (pairs, excluded pairs and PME) and empty
+// the accumulator.  One launch and 32 bytes a place less than a gather and a
+// finish.  Without `accumulate` every atom is written: those with no place (a
+// position that was not finite at the build) get zeros.
+template <int P, bool FIXED>
+__global__ void __launch_bounds__(128) nb_finish_gather(GridParams G, int64_t places, int64_t n,
+                                                        const int32_t *__restrict__ sizes,
+                                                        const int32_t *__restrict__ order,
+                                                        const int32_t *__restrict__ place_of,
+                                                        const float4 *__restrict__ xq, const float *__restrict__ phi,
+                                                        float4 *__restrict__ acc,
+                                                        unsigned long long *__restrict__ accf,
+                                                        double *__restrict__ forces, int accumulate,
+                                                        float *__restrict__ pot) {
+  int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  int64_t p = t / P;
+  int c = (int)(t & (P - 1));
+  if (!accumulate && c == 0 && p < n && sizes[NB_SIZE_NAN] > 0 && place_of[p] < 0)
+    forces[3 * p] = forces[3 * p + 1] = forces[3 * p + 2] = 0.0;
+  bool live = p < places && p < sizes[NB_SIZE_PLACES];
+  int a = live ? order[p] : -1;
+  float g0 = 0.f, g1 = 0.f, g2 = 0.f, e = 0.f;
+  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (a >= 0) {
+    v = xq[p];
+    int k0, k1, k2;
+    float t0, t1, t2;
+    nb_frac3(v, G, k0, k1, k2, t0, t1, t2);
+    float w0[P], w1[P], w2[P], d0[P], d1[P], d2[P];
+    nb_bspline<P>(t0, w0, d0);
+    nb_bspline<P>(t1, w1, d1);
+    nb_bspline<P>(t2, w2, d2);
+    int gz = k2 - c;
+    if (gz < 0) gz += G.K2;
+    float wz = nb_pick(w2, c), dz = nb_pick(d2, c);
+#pragma unroll
+    for (int jx = 0; jx < P; ++jx) {
+      int gx = k0 - jx;
+      if (gx < 0) gx += G.K0;
+#pragma unroll
+      for (int jy = 0; jy < P; ++jy) {
+        int gy = k1 - jy;
+        if (gy < 0) gy += G.K1;
+        float f = __ldg(phi + ((int64_t)gx * G.K1 + gy) * G.K2 + gz);
+        float wxy = w0[jx] * w1[jy];
+        g0 = fmaf(d0[jx] * w1[jy], f, g0);
+        g1 = fmaf(w0[jx] * d1[jy], f, g1);
+        e = fmaf(wxy, f, e);
+        g2 = fmaf(wxy, f, g2);
+      }
+    }
+    g0 *= wz;
+    g1 *= wz;
+    g2 *= dz;
+    e *= wz;
+  }
+#pragma unroll
+  for (int o = P / 2; o > 0; o >>= 1) {
+    g0 += __shfl_xor_sync(0xffffffffu, g0, o);
+    g1 += __shfl_xor_sync(0xffffffffu, g1, o);
+    g2 += __shfl_xor_sync(0xffffffffu, g2, o);
+    e += __shfl_xor_sync(0xffffffffu, e, o);
+  }
+  if (!live) return;
+  if (pot && c == 0) pot[p] = e;
+  if (c >= 3) return;
+  const float3 F = nb_frac_force(G, v.w, g0, g1, g2);
+  double f;
+  if (FIXED) {
+    f = (double)(long long)accf[3 * p + c] * NB_FORCE_SCALE_INV;
+    accf[3 * p + c] = 0ull;
+  } else {
+    float *at = reinterpret_cast<float *>(acc + p) + c;
+    f = (double)*at;
+    *at = 0.f;
+  }
+  if (a < 0) return;
+  f += (double)(c == 0 ? F.x : c == 1 ? F.y : F.z);
+  double *out = forces + 3 * (int64_t)a + c;
+  *out = accumulate ? *out + f : f;
+}
+
 // The adjoint of the reciprocal forces for the force-matching product.
 // With Q = sum_j q_j W_j, phi = Psi * Q and F_i = -q_i sum_k phi(k) grad W_i(k):
 //   sum_i g_i . dF_i/dq_m = -g_m . sum_k phi(k) grad W_m(k) - sum_k W_m(k) psi(k),
@@ -1167,7 +1251,11 @@ int nb_pme_setup(NbCtx &c, int k0, int k1, int k2, int order) {
   P.order = order;
   int64_t total = (int64_t)k0 * k1 * k2;
   int64_t half = (int64_t)k0 * k1 * (k2 / 2 + 1);
-  if (cudaMalloc(&P.grid, sizeof(float) * total) != cudaSuccess) return -1;
+  if (cudaMalloc(&P.grid, sizeof(float) * total) != cudaSuccess ||
+      cudaMalloc(&P.phi, sizeof(float) * total) != cudaSuccess)
+    return -1;
+  cudaMemset(P.grid, 0, sizeof(float) * total);
+  cudaMemset(P.phi, 0, sizeof(float) * total);
   if (cudaMalloc(&P.spec, sizeof(float2) * half) != cudaSuccess) return -1;
   if (cudaMalloc(&P.fixed, sizeof(unsigned long long) * total) != cudaSuccess) return -1;
   cudaMemset(P.fixed, 0, sizeof(unsigned long long) * total);
@@ -1222,7 +1310,7 @@ void nb_pme_release(NbCtx &c) {
   if (P.fwd) cufftDestroy(P.fwd);
   if (P.bwd) cufftDestroy(P.bwd);
   P.fwd = P.bwd = 0;
-  for (void *p : {(void *)P.grid, (void *)P.spec, (void *)P.fixed, (void *)P.moduli,
+  for (void *p : {(void *)P.grid, (void *)P.phi, (void *)P.spec, (void *)P.fixed, (void *)P.moduli,
                   (void *)P.pme_force, (void *)P.potential, (void *)P.partials, (void *)P.adj_grid,
                   (void *)P.influence, (void *)P.fft_tw, (void *)P.tile_count, (void *)P.tile_start,
                   (void *)P.tile_scratch, (void *)P.tile_bin, (void *)P.tile_rank, (void *)P.tile_sorted})
@@ -1233,6 +1321,7 @@ void nb_pme_release(NbCtx &c) {
   P.adj_grid = nullptr;
   P.influence = nullptr;
   P.grid = nullptr;
+  P.phi = nullptr;
   P.spec = nullptr;
   P.fixed = nullptr;
   P.moduli = nullptr;
@@ -1282,7 +1371,7 @@ static void nb_pme_sums(NbCtx &c, int rows, cudaStream_t s) {
                                                                    nb_done_blocks(c) + 1);
 }
 
-int nb_pme_run(NbCtx &c, const double box[3], bool energy, bool potential, cudaStream_t s) {
+int nb_pme_run(NbCtx &c, const double box[3], bool energy, bool potential, cudaStream_t s, bool gather) {
   NbPme &P = c.pme;
   if (!P.on) return 0;
   GridParams G;
@@ -1295,7 +1384,6 @@ int nb_pme_run(NbCtx &c, const double box[3], bool energy, bool potential, cudaS
   nb_cell_tilts(c, box, G, nullptr);
   int64_t total = (int64_t)G.K0 * G.K1 * G.K2;
   int64_t half = (int64_t)G.K0 * G.K1 * (G.K2 / 2 + 1);
-  if (!c.deterministic) cudaMemsetAsync(P.grid, 0, sizeof(float) * total, s);
   nb_spread_run(c, G, P.grid, P.fixed, nullptr, s);
   bool own = nb_fft_own(c);
   if (c.deterministic && !own) nb_fixed_to_grid<<<blocks_for((total + 3) / 4, 256), 256, 0, s>>>(total, P.fixed, P.grid);
@@ -1311,9 +1399,10 @@ int nb_pme_run(NbCtx &c, const double box[3], bool energy, bool potential, cudaS
   C.pi2_beta2 = M_PI * M_PI / (c.beta * c.beta);
   nb_cell_tilts(c, box, G, &C);
   if (own) {
-    // spread grid -> potential in P.grid, the fixed-point grid read directly
+    // spread grid -> potential, the fixed-point grid read directly; the grid it
+    // read is empty again
     if (!energy && nb_pme_table(c, box, s)) return -1;
-    if (nb_fft_convolve(P, P.grid, c.deterministic ? P.fixed : nullptr, P.spec, P.grid, P.influence, energy, C,
+    if (nb_fft_convolve(P, P.grid, c.deterministic ? P.fixed : nullptr, P.spec, P.phi, P.influence, energy, C,
                         P.partials, nullptr, s))
       return -3;
     if (energy) nb_pme_sums(c, (int)nb_fft_column_blocks(P.K), s);
@@ -1323,23 +1412,51 @@ int nb_pme_run(NbCtx &c, const double box[3], bool energy, bool potential, cudaS
     if (cufftExecR2C(P.fwd, P.grid, (cufftComplex *)P.spec) != CUFFT_SUCCESS) return -3;
     if (energy) {
       nb_convolve<true><<<blocks_for(half, 256), 256, 0, s>>>(C, P.moduli, P.spec, P.partials);
+      cudaMemsetAsync(P.grid, 0, sizeof(float) * total, s);  // empty for the next spreading
       nb_pme_sums(c, P.conv_blocks, s);
     } else {
       if (nb_pme_table(c, box, s)) return -1;
-      nb_scale_spectrum<<<blocks_for(half, 256), 256, 0, s>>>(half, P.influence, P.spec, nullptr, 0, nullptr);
+      nb_scale_spectrum<<<blocks_for(half, 256), 256, 0, s>>>(half, P.influence, P.spec, P.grid, total, nullptr);
     }
-    if (cufftExecC2R(P.bwd, (cufftComplex *)P.spec, P.grid) != CUFFT_SUCCESS) return -3;
+    if (cufftExecC2R(P.bwd, (cufftComplex *)P.spec, P.phi) != CUFFT_SUCCESS) return -3;
   }
+  if (!gather) return 0;
   float *pot = potential ? P.potential : nullptr;
   int blocks = blocks_for(c.places_cap, 128);
   float4 *pf = (float4 *)P.pme_force;
   switch (P.order) {
-    case 4: nb_pme_gather_split<4><<<blocks_for(c.places_cap * 4, 128), 128, 0, s>>>(G, c.places_cap, c.sizes, c.order, c.xq, P.grid, pf, pot); break;
-    case 5: nb_pme_gather<5><<<blocks, 128, 0, s>>>(G, c.places_cap, c.sizes, c.order, c.xq, P.grid, pf, pot); break;
-    case 6: nb_pme_gather<6><<<blocks, 128, 0, s>>>(G, c.places_cap, c.sizes, c.order, c.xq, P.grid, pf, pot); break;
-    case 8: nb_pme_gather_split<8><<<blocks_for(c.places_cap * 8, 128), 128, 0, s>>>(G, c.places_cap, c.sizes, c.order, c.xq, P.grid, pf, pot); break;
+    case 4: nb_pme_gather_split<4><<<blocks_for(c.places_cap * 4, 128), 128, 0, s>>>(G, c.places_cap, c.sizes, c.order, c.xq, P.phi, pf, pot); break;
+    case 5: nb_pme_gather<5><<<blocks, 128, 0, s>>>(G, c.places_cap, c.sizes, c.order, c.xq, P.phi, pf, pot); break;
+    case 6: nb_pme_gather<6><<<blocks, 128, 0, s>>>(G, c.places_cap, c.sizes, c.order, c.xq, P.phi, pf, pot); break;
+    case 8: nb_pme_gather_split<8><<<blocks_for(c.places_cap * 8, 128), 128, 0, s>>>(G, c.places_cap, c.sizes, c.order, c.xq, P.phi, pf, pot); break;
   }
   return 0;
+}
+
+bool nb_finish_gathers(const NbCtx &c) { return c.pme.order == 4 || c.pme.order == 8; }
+
+void nb_finish_gather_run(NbCtx &c, const double box[3], double *forces, int accumulate, bool potential,
+                          cudaStream_t s) {
+  NbPme &P = c.pme;
+  GridParams G;
+  G.K0 = P.K[0];
+  G.K1 = P.K[1];
+  G.K2 = P.K[2];
+  G.invL0 = (float)(1.0 / box[0]);
+  G.invL1 = (float)(1.0 / box[1]);
+  G.invL2 = (float)(1.0 / box[2]);
+  nb_cell_tilts(c, box, G, nullptr);
+  float *pot = potential ? P.potential : nullptr;
+#define NB_FINISH_GATHER(ORD, F)                                                                                     \
+  nb_finish_gather<ORD, F><<<blocks_for(c.places_cap * ORD, 128), 128, 0, s>>>(G, c.places_cap, c.n, c.sizes, c.order, \
+                                                                              c.place_of, c.xq, P.phi, c.acc,        \
+                                                                              c.acc_fixed, forces, accumulate, pot)
+  if (P.order == 4) {
+    if (c.deterministic) NB_FINISH_GATHER(4, true); else NB_FINISH_GATHER(4, false);
+  } else {
+    if (c.deterministic) NB_FINISH_GATHER(8, true); else NB_FINISH_GATHER(8, false);
+  }
+#undef NB_FINISH_GATHER
 }
 
 // The reciprocal part of the parameter gradient in the charges, added per
@@ -1361,9 +1478,9 @@ int nb_pme_adjoint_run(NbCtx &c, const double box[3], int mode, cudaStream_t s, 
   int64_t half = (int64_t)G.K0 * G.K1 * (G.K2 / 2 + 1);
   if (!P.adj_grid && cudaMalloc(&P.adj_grid, sizeof(float) * total) != cudaSuccess) return -2;
   if (!phi) {
-    int rc = nb_pme_run(c, box, false, false, s);  // phi in P.grid
+    int rc = nb_pme_run(c, box, false, false, s, false);
     if (rc) return rc;
-    phi = P.grid;
+    phi = P.phi;
   }
   int blocks = blocks_for(c.places_cap, 128);
   if (mode == 1) {
@@ -1755,13 +1872,13 @@ int nb_batch_pme_run(mdrtNbBatch &b, bool energy, cudaStream_t s) {
   return 0;
 }
 
-// The potential grid of the last force evaluation (K0 K1 K2 f32, in P.grid)
+// The potential grid of the last force evaluation (K0 K1 K2 f32)
 // to `out` (device), on s.
 int nb_pme_potential_grid(NbCtx &c, float *out, cudaStream_t s) {
   NbPme &P = c.pme;
   if (!P.on) return -2;
   int64_t total = (int64_t)P.K[0] * P.K[1] * P.K[2];
-  return cudaMemcpyAsync(out, P.grid, sizeof(float) * total, cudaMemcpyDeviceToDevice, s) == cudaSuccess ? 0 : -1;
+  return cudaMemcpyAsync(out, P.phi, sizeof(float) * total, cudaMemcpyDeviceToDevice, s) == cudaSuccess ? 0 : -1;
 }
 
 // ---------------------------------------------------------------------------
