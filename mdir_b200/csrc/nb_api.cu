@@ -256,6 +256,11 @@ int32_t mdrtNbSetParticles(mdrtNb *ctx, const double *charges, const int32_t *ty
   for (int64_t i = 0; i < c.n; ++i)
     if (types[i] < 0 || types[i] >= ntypes || !std::isfinite(charges[i])) return MDRT_NB_INVALID_ARGUMENT;
   c.h_q.assign(charges, charges + c.n);
+  ctx->q_sum = ctx->q_sq = 0.0;
+  for (double v : c.h_q) {
+    ctx->q_sq += v * v;
+    ctx->q_sum += v;
+  }
   const bool same_types = (int64_t)c.h_type.size() == c.n && std::equal(c.h_type.begin(), c.h_type.end(), types);
   c.h_type.assign(types, types + c.n);
   c.h_lj.resize((size_t)ntypes * ntypes);
@@ -674,8 +679,8 @@ int32_t mdrtNbParameterGradientFrames(mdrtNb *ctx, const double *x, int64_t x_st
   int32_t ready = nb_gradient_ready(ctx, x, box, cotangent, mode, potentials, dq, dtable, stream);
   if (ready) return ready;
   auto run = [&](cudaStream_t s) -> int32_t {
-    if (nb_adjoint_run(ctx->c, x, x_stride, count, box, cotangent, c_stride, mode, potentials, p_stride, dq, dtable,
-                       s))
+    if (nb_adjoint_run(ctx->c, x, x_stride, count, box, cotangent, c_stride, mode, potentials, p_stride, ctx->q_sum,
+                       dq, dtable, s))
       return MDRT_NB_CUDA_ERROR;
     CK(cudaGetLastError());
     return MDRT_NB_OK;
@@ -776,7 +781,8 @@ int32_t mdrtNbParameterGradientPotential(mdrtNb *ctx, const double *x, const dou
                                          double *dtable, void *stream) {
   int32_t s = nb_gradient_ready(ctx, x, box, cotangent, mode, phi, dq, dtable, stream);
   if (s) return s;
-  if (nb_adjoint_run(ctx->c, x, 0, 1, box, cotangent, 0, mode, phi, 0, dq, dtable, (cudaStream_t)stream))
+  if (nb_adjoint_run(ctx->c, x, 0, 1, box, cotangent, 0, mode, phi, 0, ctx->q_sum, dq, dtable,
+                     (cudaStream_t)stream))
     return MDRT_NB_CUDA_ERROR;
   CK(cudaGetLastError());
   return MDRT_NB_OK;
@@ -795,11 +801,7 @@ int32_t mdrtNbEnergies(mdrtNb *ctx, void *stream, double *out) {
 int32_t mdrtNbConstants(mdrtNb *ctx, const double box[3], int32_t dispersion, double *out) {
   if (!ctx || !box || !out) return MDRT_NB_INVALID_ARGUMENT;
   NbCtx &c = ctx->c;
-  double sq = 0.0, net = 0.0;
-  for (double v : c.h_q) {
-    sq += v * v;
-    net += v;
-  }
+  const double sq = ctx->q_sq, net = ctx->q_sum;
   double V = box[0] * box[1] * box[2];
   out[0] = c.beta > 0 ? -c.coulomb * c.beta / std::sqrt(M_PI) * sq : 0.0;
   out[1] = c.beta > 0 ? -c.coulomb * M_PI * net * net / (2.0 * V * c.beta * c.beta) : 0.0;

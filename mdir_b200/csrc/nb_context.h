@@ -190,6 +190,9 @@ struct mdrtNb {
   NbCtx c;
   std::vector<NbFrameGraph> graphs;
   uint64_t graph_clock = 0;
+  // the sums of the charges and of their squares, in atom order, as the
+  // particles were set; kept out of NbCtx like the charges themselves
+  double q_sum = 0.0, q_sq = 0.0;
   // the reciprocal chain of a force call runs on `side` beside its pairs
   cudaStream_t side = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
@@ -238,6 +241,7 @@ struct mdrtNbBatch {
   int64_t groups_alloc = 0, cols_alloc = 0;
   int32_t *frame_units = nullptr; // per frame: first unit, one past the last
   std::vector<double> h_boxes;    // frames x 3 of the last build
+  std::vector<double> h_q;        // frames x 2: each frame's sums of the charges and of their squares
   // excluded pairs: blocks of 256 pairs that never straddle two frames
   int32_t *excl_blk_frame = nullptr, *excl_blk_first = nullptr, *excl_frame_end = nullptr;
   std::vector<int32_t> h_excl_blk0;  // frames + 1
@@ -349,11 +353,12 @@ void nb_finish_gather_run(NbCtx &c, const double box[3], double *forces, int acc
 // g (f64 [n,3], atom order); mode 1: dE/dtheta.  Adds the charge gradient to
 // dq (f64 [n], atom order) and the type-pair gradient to dtable (f64,
 // ntypes^2 sigma entries then ntypes^2 epsilon entries), each reduced once
-// at the end of the call.  Needs the adjoint scratch (nb_adjoint_reserve).
+// at the end of the call.  `net`: the sum of the charges (mode 1).  Needs the
+// adjoint scratch (nb_adjoint_reserve).
 int nb_adjoint_reserve(NbCtx &c, cudaStream_t s);
 int nb_adjoint_run(NbCtx &c, const double *x, int64_t x_stride, int64_t count, const double box[3],
                    const double *cotangent, int64_t c_stride, int mode, const float *phi, int64_t p_stride,
-                   double *dq, double *dtable, cudaStream_t s);
+                   double net, double *dq, double *dtable, cudaStream_t s);
 // The reciprocal part of the charge gradient, added per place into c.adj_q.
 int nb_pme_potential_grid(NbCtx &c, float *out, cudaStream_t s);
 // With phi (a potential grid kept from the force evaluation at the same

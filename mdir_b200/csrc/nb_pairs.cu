@@ -1290,8 +1290,8 @@ int nb_adjoint_reserve(NbCtx &c, cudaStream_t s) {
 }
 
 int nb_adjoint_run(NbCtx &c, const double *x, int64_t x_stride, int64_t count, const double box[3],
-                   const double *cot, int64_t c_stride, int mode, const float *phi, int64_t p_stride, double *dq,
-                   double *dtable, cudaStream_t s) {
+                   const double *cot, int64_t c_stride, int mode, const float *phi, int64_t p_stride, double net,
+                   double *dq, double *dtable, cudaStream_t s) {
   PairParams P = pair_params(c, box);
   bool inner = c.inner_reach > 0.0 && c.inner_valid;
   const int32_t *lsizes = inner ? c.sizes_in : c.sizes;
@@ -1307,9 +1307,6 @@ int nb_adjoint_run(NbCtx &c, const double *x, int64_t x_stride, int64_t count, c
   // the blocks' type-pair partials and the places' charge gradient (kept
   // zero between calls) sum the frames; both go out once at the end
   if (cudaMemsetAsync(c.adj_types, 0, sizeof(double) * grid * width, s) != cudaSuccess) return -1;
-  double net = 0.0;
-  if (mode == 1)
-    for (double v : c.h_q) net += v;
   for (int64_t k = 0; k < count; ++k) {
     const double *xk = x + k * x_stride;
     const double *ck = mode == 0 ? cot + k * c_stride : nullptr;

@@ -38,3 +38,17 @@ def test_energies_are_the_oracles_and_reproducible(cuda, waters):
     scale = sum(abs(ref[k]) for k in ("lj", "coulomb", "excluded"))
     for value, k in zip(seen[0], ("lj", "coulomb", "excluded")):
         assert abs(value - ref[k]) <= 1e-6 * scale
+
+
+def test_batch_constants_follow_the_charges(cuda):
+    from mdir_b200 import systems
+    from mdir_b200.batch import BatchEvaluator
+    frames = systems.batch_frames(count=5, low=1000, high=2000, seed=8)
+    ev = BatchEvaluator(frames)
+    ev.force(energy=True)
+    e = ev.energies()
+    for k, f in enumerate(frames):
+        q = np.asarray(f["charges"])
+        want = -systems.COULOMB * f["beta"] / np.sqrt(np.pi) * np.sum(q * q)
+        assert abs(e["self"][k] - want) <= 1e-12 * abs(want)
+    ev.close()
