@@ -607,11 +607,16 @@ __device__ void md_last_block(const UpdateParams &U, const double *ke_part, cons
   if (U.check_build) {
     // the drift the lists may reach before the next decision: its growth
     // over the window just ended, once more (thermo[6] holds the drift at
-    // the last decision, 0 after a build; the largest drift grows slower
-    // than the first, ballistic, window); a wrong guess is caught by the test
-    // of every step and costs a redo, not a missed pair
+    // the last decision, 0 after a build); a wrong guess is caught by the test
+    // of every step and costs a redo, not a missed pair.  The first window
+    // after a build is ballistic (every atom at its own speed from its
+    // reference), and the largest drift grows slower after it, so its growth
+    // counts two thirds (the default of 1.5 becomes 1: no further than as fast
+    // again): with skins near 2.5 first windows (0.25 nm half skin) the full
+    // factor asked for a build at every decision.
     double d = sqrt((double)d2);
-    double ahead = d + U.lookahead * fmax(d - thermo[6], 0.0) + 0.002;
+    double factor = thermo[6] == 0.0 ? U.lookahead * (2.0 / 3.0) : U.lookahead;
+    double ahead = d + factor * fmax(d - thermo[6], 0.0) + 0.002;
     rebuild = (stale || ahead * ahead > U.build_half2) ? 1 : 0;
     thermo[6] = d;
     stale = 0;
