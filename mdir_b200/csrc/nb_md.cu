@@ -1262,7 +1262,7 @@ static int32_t md_prepare_graph(mdrtMd *m, double *x, double *v, const double bo
     cudaStreamCreateWithFlags(&body, cudaStreamNonBlocking);
     cudaError_t e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
     m->handles.assign(1, 0);
-    if (e == cudaSuccess)
+    if (e == cudaSuccess && m->tau > 0.0)  // no thermostat reads no noise
       md_noise<<<(unroll + 31) / 32, 32, 0, cap>>>(m->thermo, m->noise, unroll, (double)m->ndof, m->seed);
     for (int k = 0; k < unroll && e == cudaSuccess; ++k) {
       bool last = k == unroll - 1;

@@ -104,6 +104,14 @@ __device__ __forceinline__ void nb_pair_terms(const PairParams &P, float r2, flo
   float rinv = nb_rsqrt(r2);
   float rinv2 = rinv * rinv;
   float s6 = rinv2 * rinv2 * rinv2;
+  if (!ENERGY && SWITCH == 0) {
+    // forces alone: one product by 1/r^2 for both terms
+    float ex = nb_ex2(r2 * P.nb2_log2e);
+    float erfcv = nb_erfc_from_exp(P.beta_p * (r2 * rinv), ex);
+    fs = rinv2 * fmaf(qq, fmaf(erfcv, rinv, P.two_beta_sqrtpi * ex), s6 * fmaf(cc.y, s6, -cc.x));
+    ulj = uc = 0.f;
+    return;
+  }
   float a12 = cc.y * s6 * s6, a6 = cc.x * s6;  // 12 c12 / r^12, 6 c6 / r^6
   fs = (a12 - a6) * rinv2;
   ulj = (ENERGY || SWITCH) ? a12 * (1.f / 12.f) - a6 * (1.f / 6.f) : 0.f;
@@ -207,7 +215,72 @@ __device__ __forceinline__ void nb_pair_unit(const PairParams &P, int2 uo, int64
   float ax = 0.f, ay = 0.f, az = 0.f;  // the accumulator of member (lane + k) mod 16
   float elj = 0.f, ecl = 0.f;
   float vxx = 0.f, vyy = 0.f, vzz = 0.f, vxy = 0.f, vxz = 0.f, vyz = 0.f;
-  for (int r = 0; r < 2; ++r) {
+  // Two dense rounds at once (the force forms): the lane holds a partner of
+  // each, a member's position and factors are read once for both, its
+  // accumulator moves on once, and the two chains of a step interleave.
+  bool both = false;
+  if (!ENERGY && !FIXED && ne > 32) {
+    const bool second = 32 + lane < ne;
+    const unsigned m0 = (unsigned)pre0.y & 0xffffu, m1 = second ? (unsigned)pre1.y & 0xffffu : 0u;
+    both = !__all_sync(FULL, __popc(m0) <= NB_SPARSE_BITS) && !__all_sync(FULL, __popc(m1) <= NB_SPARSE_BITS);
+    if (both) {
+      NbCell H;
+      H.ax = Lx;
+      H.by = Ly;
+      H.cz = Lz;
+      H.bx = P.bx;
+      H.cx = P.cx;
+      H.cy = P.cy;
+      auto partner = [&](int q, int bits, int &tj, float2 &fj) {
+        float4 xj = xq[q];
+        tj = typ[q];
+        int sx, sy, sz;
+        nb_decode_image(((unsigned)bits >> 16) & NB_IMAGE_BITS, sx, sy, sz);
+        const float3 t = nb_lattice_shift(sx, sy, sz, H);
+        xj.x += t.x;
+        xj.y += t.y;
+        xj.z += t.z;
+        fj = LJM == 1 ? ljf[tj] : make_float2(0.f, 0.f);
+        return xj;
+      };
+      const int q0 = pre0.x, q1 = second ? pre1.x : 0;
+      int t0, t1;
+      float2 f0, f1;
+      const float4 x0 = partner(q0, pre0.y, t0, f0);
+      const float4 x1 = partner(q1, second ? pre1.y : 0, t1, f1);
+      const unsigned rot0 = (m0 >> u) | (m0 << (16 - u)), rot1 = (m1 >> u) | (m1 << (16 - u));
+      float3 j0 = make_float3(0.f, 0.f, 0.f), j1 = j0;
+#pragma unroll
+      for (int k = 0; k < NB_GROUP; ++k) {
+        const float4 xm = s_xw[u + k];
+        const float2 fm = LJM == 1 ? s_fw[u + k] : make_float2(0.f, 0.f);
+        const int tm = LJM == 1 ? 0 : s_tw[u + k];
+        auto one = [&](const float4 &xj, const float2 &fj, int tj, unsigned rot, float3 &j) {
+          const float dx = xm.x - xj.x, dy = xm.y - xj.y, dz = xm.z - xj.z;
+          const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+          const bool inside = (rot & (1u << k)) != 0u && r2 < P.rc2;
+          const float2 cc = LJM == 1 ? make_float2(fm.x * fj.x, fm.y * fj.y) : s_lj[tm + tj];
+          float fs, ulj, uc;
+          nb_pair_terms<ENERGY, SWITCH>(P, r2, cc, xm.w * xj.w, fs, ulj, uc);
+          fs = inside ? fs : 0.f;
+          j.x = fmaf(-fs, dx, j.x);
+          j.y = fmaf(-fs, dy, j.y);
+          j.z = fmaf(-fs, dz, j.z);
+          ax = fmaf(fs, dx, ax);
+          ay = fmaf(fs, dy, ay);
+          az = fmaf(fs, dz, az);
+        };
+        one(x0, f0, t0, rot0, j0);
+        one(x1, f1, t1, rot1, j1);
+        ax = __shfl_sync(FULL, ax, src);
+        ay = __shfl_sync(FULL, ay, src);
+        az = __shfl_sync(FULL, az, src);
+      }
+      if (j0.x != 0.f || j0.y != 0.f || j0.z != 0.f) nb_red_add_v4(acc + q0, j0.x, j0.y, j0.z);
+      if (j1.x != 0.f || j1.y != 0.f || j1.z != 0.f) nb_red_add_v4(acc + q1, j1.x, j1.y, j1.z);
+    }
+  }
+  for (int r = both ? 2 : 0; r < 2; ++r) {
     if (r * 32 >= ne) break;
     bool valid = r * 32 + lane < ne;
     int2 en = valid ? ((ENERGY && !STAGED) ? row[r * 32 + lane] : (r == 0 ? pre0 : pre1)) : make_int2(0, 0);
