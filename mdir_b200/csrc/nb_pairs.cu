@@ -214,7 +214,26 @@ __device__ __forceinline__ void nb_pair_unit(const PairParams &P, int2 uo, int64
   }
   float ax = 0.f, ay = 0.f, az = 0.f;  // the accumulator of member (lane + k) mod 16
   float elj = 0.f, ecl = 0.f;
+  // The virial sum of d f over the unit's pairs from its sums of forces: each
+  // member's and partner's place, less the group's first, times the force the
+  // unit puts on it (the places lie within the reach of that one, so nothing is
+  // lost to the size of the cell).  Six products an entry instead of six a slot.
   float vxx = 0.f, vyy = 0.f, vzz = 0.f, vxy = 0.f, vxz = 0.f, vyz = 0.f;
+  auto virial = [&](float4 x, float3 lo, float fx, float fy, float fz) {
+    const float4 c = s_xw[0];
+    float dx = x.x - c.x, dy = x.y - c.y, dz = x.z - c.z;
+    if (FIXED) {
+      dx += lo.x;
+      dy += lo.y;
+      dz += lo.z;
+    }
+    vxx = fmaf(dx, fx, vxx);
+    vyy = fmaf(dy, fy, vyy);
+    vzz = fmaf(dz, fz, vzz);
+    vxy = fmaf(dx, fy, vxy);
+    vxz = fmaf(dx, fz, vxz);
+    vyz = fmaf(dy, fz, vyz);
+  };
   // Two dense rounds at once (the force forms): the lane holds a partner of
   // each, a member's position and factors are read once for both, its
   // accumulator moves on once, and the two chains of a step interleave.
@@ -351,12 +370,6 @@ __device__ __forceinline__ void nb_pair_unit(const PairParams &P, int2 uo, int64
       if (ENERGY) {
         elj += inside ? ulj : 0.f;
         ecl += inside ? uc : 0.f;
-        vxx = fmaf(dx, fx, vxx);
-        vyy = fmaf(dy, fy, vyy);
-        vzz = fmaf(dz, fz, vzz);
-        vxy = fmaf(dx, fy, vxy);
-        vxz = fmaf(dx, fz, vxz);
-        vyz = fmaf(dy, fz, vyz);
       }
     };
     if (__all_sync(FULL, __popc(mask) <= NB_SPARSE_BITS)) {
@@ -421,6 +434,7 @@ __device__ __forceinline__ void nb_pair_unit(const PairParams &P, int2 uo, int64
         az = __shfl_sync(FULL, az, src);
       }
     }
+    if (ENERGY) virial(xj, jl, fjx, fjy, fjz);
     if (valid && (fjx != 0.f || fjy != 0.f || fjz != 0.f)) {
       if (FIXED)
         nb_red_fixed(accf + 3 * (int64_t)q, fjx, fjy, fjz, status);
@@ -436,6 +450,10 @@ __device__ __forceinline__ void nb_pair_unit(const PairParams &P, int2 uo, int64
       nb_red_fixed(accf + 3 * pi, ax, ay, az, status);
     else
       nb_red_add_v4(acc + pi, ax, ay, az);
+  }
+  if (ENERGY && lane < 16) {
+    const float4 lo = FIXED ? s_lw[u] : make_float4(0.f, 0.f, 0.f, 0.f);
+    virial(s_xw[u], make_float3(lo.x, lo.y, lo.z), ax, ay, az);
   }
   if (ENERGY) {
     double v[8] = {elj, ecl, vxx, vyy, vzz, vxy, vxz, vyz};
