@@ -238,12 +238,6 @@ __device__ __forceinline__ float4 md_frame(int p, Vec3 x, char4 s, const double 
   return nf;
 }
 
-__device__ __forceinline__ float4 write_frame(int p, Vec3 x, const char4 *__restrict__ shift, const double *L,
-                                              float4 *xq, float4 *xq_lo) {
-  if (p < 0) return make_float4(0.f, 0.f, 0.f, 0.f);
-  return md_frame(p, x, shift[p], L, xq[p].w, xq, xq_lo);
-}
-
 // The PME force on the atom at frame fr (charge fr.w), gathered from the
 // potential grid with order-4 B-splines: F = -q sum_k phi(k) grad W(k).
 __device__ __forceinline__ Vec3 md_pme_gather(float4 fr, const float *__restrict__ phi, const GridParams &G) {
@@ -437,25 +431,27 @@ __global__ void __launch_bounds__(MD_UPDATE_THREADS) md_update(
     int64_t t = (int64_t)(blockIdx.x - water_blocks) * blockDim.x + threadIdx.x;
     int i = free_atoms[t];
     int pi = fplace[t];
+    // as the waters: every load of data that no kernel of this step writes,
+    // and the PME gather, before the wait
+    Vec3 xi = load3(x, i), vi = load3(v, i), xr = load3(x_ref, i);
+    const double im = inv_mass[i], ms = mass[i];
+    const char4 sh = pi >= 0 ? shift[pi] : make_char4(0, 0, 0, 0);
+    const float4 fr = pi >= 0 ? xq[pi] : make_float4(0.f, 0.f, 0.f, 0.f);
     Vec3 fg = {0.0, 0.0, 0.0};
-    bool gather = false;
-    if (U.pme_fused && pi >= 0) {
-      float4 fr = xq[pi];
-      gather = fr.w != 0.f;
-      if (gather) fg = md_pme_gather(fr, U.phi, U.G);
-    }
+    const bool gather = U.pme_fused && pi >= 0 && fr.w != 0.f;
+    if (gather) fg = md_pme_gather(fr, U.phi, U.G);
     nb_grid_wait();
     if (halt) return;
     Vec3 fi = take_force(pi, acc, accf, pme, U.fixed);
     if (gather) fi = fi + fg;
-    Vec3 vi = lambda * load3(v, i) + (dt * inv_mass[i]) * fi;
-    Vec3 xi = load3(x, i) + dt * vi;
+    vi = lambda * vi + (dt * im) * fi;
+    xi = xi + dt * vi;
     store3(x, i, xi);
     store3(v, i, vi);
     store3(fout, i, fi);
-    write_frame(pi, xi, shift, U.L, xq, xq_lo);
-    ke = 0.5 * mass[i] * dot(vi, vi);
-    Vec3 di = xi - load3(x_ref, i);
+    if (pi >= 0) md_frame(pi, xi, sh, U.L, fr.w, xq, xq_lo);
+    ke = 0.5 * ms * dot(vi, vi);
+    Vec3 di = xi - xr;
     d2max = (float)dot(di, di);
     if (U.prune_half2 > 0.0) {
       di = xi - load3(x_prune, i);
