@@ -173,7 +173,7 @@ __device__ __forceinline__ void nb_pair_unit(const PairParams &P, int2 uo, int64
                                              const float2 *s_lj, float4 *s_xw, float2 *s_fw, int *s_tw,
                                              float (*s_bw)[NB_SPARSE_BITS][33], float4 *__restrict__ acc,
                                              unsigned long long *__restrict__ accf, double *__restrict__ partials,
-                                             int *__restrict__ status) {
+                                             int *__restrict__ status, int first = 0, int last = 2) {
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31, u = lane & 15;
   const int src = (lane & 16) | ((lane + 1) & 15);  // the lane the member accumulators come from
@@ -238,7 +238,7 @@ __device__ __forceinline__ void nb_pair_unit(const PairParams &P, int2 uo, int64
   // each, a member's position and factors are read once for both, its
   // accumulator moves on once, and the two chains of a step interleave.
   bool both = false;
-  if (!ENERGY && !FIXED && ne > 32) {
+  if (!ENERGY && !FIXED && ne > 32 && first == 0 && last == 2) {
     const bool second = 32 + lane < ne;
     const unsigned m0 = (unsigned)pre0.y & 0xffffu, m1 = second ? (unsigned)pre1.y & 0xffffu : 0u;
     both = !__all_sync(FULL, __popc(m0) <= NB_SPARSE_BITS) && !__all_sync(FULL, __popc(m1) <= NB_SPARSE_BITS);
@@ -299,7 +299,7 @@ __device__ __forceinline__ void nb_pair_unit(const PairParams &P, int2 uo, int64
       if (j1.x != 0.f || j1.y != 0.f || j1.z != 0.f) nb_red_add_v4(acc + q1, j1.x, j1.y, j1.z);
     }
   }
-  for (int r = both ? 2 : 0; r < 2; ++r) {
+  for (int r = both ? 2 : first; r < last; ++r) {
     if (r * 32 >= ne) break;
     bool valid = r * 32 + lane < ne;
     int2 en = valid ? ((ENERGY && !STAGED) ? row[r * 32 + lane] : (r == 0 ? pre0 : pre1)) : make_int2(0, 0);
@@ -552,6 +552,19 @@ __global__ void __launch_bounds__(NB_PAIR_WARPS * 32, 32 / NB_PAIR_WARPS) nb_pai
       e0 = n0;
       e1 = n1;
     }
+    return;
+  }
+  if (!ENERGY && !FIXED && 2 * nunits <= wstride) {
+    // fewer units than half the warps: a warp takes one round of 32 entries
+    // instead of two (forces alone: a unit's energies are one warp's), since a
+    // small system waits for one unit's latency (864 atoms: the MD step 13.5 ->
+    // 11.7 µs).  Not in the fixed-point mode, whose bits would follow the size
+    // of the grid.
+    if (unit < 2 * nunits)
+      nb_pair_unit<ENERGY, FIXED, SWITCH, LJM, BATCH>(
+          P, units[unit >> 1], unit >> 1, make_int2(0, 0), make_int2(0, 0), group_L, slab, counts, xq, xq_lo,
+          s_l[warp], typ, ljf, s_lj, s_x[warp], s_f[warp], s_t[warp], s_b[warp], acc, accf, partials, status,
+          unit & 1, (unit & 1) + 1);
     return;
   }
   int2 uo_next = !ENERGY && unit < nunits ? units[unit] : make_int2(0, 0);

@@ -25,8 +25,9 @@ def close(a, b, tol):
     return np.linalg.norm(a - b) <= tol * np.linalg.norm(b)
 
 
-# below and above the sizes from which the chain runs beside (2,000 atoms with energies, 6,000 without)
-@pytest.mark.parametrize("waters", [300, 1999, 2000, 2700])
+# below and above the sizes from which the chain runs beside (2,000 atoms with
+# energies, 6,000 without) and the units of a warp are whole (about 4,000)
+@pytest.mark.parametrize("waters", [300, 1300, 1999, 2000, 2700])
 @pytest.mark.parametrize("order", [4, 5, 6, 8])
 @pytest.mark.parametrize("deterministic", [False, True])
 def test_the_call_is_the_sum_of_its_parts(cuda, waters, order, deterministic):
