@@ -517,8 +517,6 @@ static int32_t nb_build_entry(mdrtNb *ctx, const double *x, int64_t n, const dou
     CK(cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming));
     CK(cudaStreamCreateWithPriority(&ctx->side, cudaStreamNonBlocking, greatest));
   }
-  if (!c.x_build) CK(cudaMalloc(&c.x_build, sizeof(double) * 3 * c.n));
-  CK(cudaMemcpyAsync(c.x_build, x, sizeof(double) * 3 * c.n, cudaMemcpyDeviceToDevice, st));
   if (sizes_out)
     for (int k = 0; k < NB_SIZE_COUNT; ++k) sizes_out[k] = c.h_sizes[k];
   if (c.h_sizes[NB_SIZE_NAN] > 0) return MDRT_NB_NAN_POSITION;

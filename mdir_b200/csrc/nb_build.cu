@@ -44,10 +44,15 @@ __global__ void nb_keys(int64_t n, const double *__restrict__ x, double Lx, doub
                         double bx, double cx, double cy,
                         int Nx, int Ny, int Nz, float inv_wx, float inv_wy, float inv_hz,
                         int32_t *__restrict__ key, int32_t *__restrict__ rank, int32_t *__restrict__ bin_count,
-                        float4 *__restrict__ atom_xw, char4 *__restrict__ atom_shift) {
+                        float4 *__restrict__ atom_xw, char4 *__restrict__ atom_shift, double *__restrict__ x_build) {
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   double v0 = x[3 * i], v1 = x[3 * i + 1], v2 = x[3 * i + 2];
+  if (x_build) {  // the positions of the build, for the displacement test
+    x_build[3 * i] = v0;
+    x_build[3 * i + 1] = v1;
+    x_build[3 * i + 2] = v2;
+  }
   bool ok = isfinite(v0) && isfinite(v1) && isfinite(v2);
   double S0 = 0, S1 = 0, S2 = 0;
   double p0 = 0, p1 = 0, p2 = 0;
@@ -690,7 +695,8 @@ __global__ void __launch_bounds__(NB_SCAN_THREADS) nb_unit_write(
   int at = nb_sum_before(block_units, blockIdx.x, sw);
   int listed = 0;
   for (int k = 0; k < NB_SCAN_PER_THREAD; ++k) {
-    const int64_t g = (int64_t)blockIdx.x * NB_SCAN_TILE + k * NB_SCAN_THREADS + threadIdx.x;
+    const int64_t g0 = (int64_t)blockIdx.x * NB_SCAN_TILE + k * NB_SCAN_THREADS, g = g0 + threadIdx.x;
+    if (g0 >= groups) break;  // the same for the block: a small system scans once
     const int n = nb_group_units(g, groups, counts, list_cap);
     int total;
     const int first = at + nb_block_exclusive_scan(n, sw, total);
@@ -953,7 +959,7 @@ static void nb_units_run(NbCtx &c, const int32_t *counts, int32_t *unit_start, i
 // search, units), two fewer where a block takes a scan alone: the small
 // kernels of a build are each a launch's latency, and 24 of them took as
 // long as the search for 900 atoms.
-static void nb_build_launch(NbCtx &c, const double *x, const double box[3], cudaStream_t s) {
+static void nb_build_launch(NbCtx &c, const double *x, const double box[3], bool keep_x, cudaStream_t s) {
   const NbGrid &G = c.grid;
   int64_t n = c.n;
   int nbins = G.nbins();
@@ -962,7 +968,7 @@ static void nb_build_launch(NbCtx &c, const double *x, const double box[3], cuda
   nb_keys<<<blocks_for(n, 256), 256, 0, s>>>(n, x, box[0], box[1], box[2], c.tilt[0], c.tilt[1], c.tilt[2],
                                             G.Nx, G.Ny, G.Nz,
                                             1.0f / G.wx, 1.0f / G.wy, 1.0f / G.hz, c.key, c.rank,
-                                            c.bin_count, c.atom_xw, c.atom_shift);
+                                            c.bin_count, c.atom_xw, c.atom_shift, keep_x ? c.x_build : nullptr);
   nb_scan(c.bin_count, c.bin_start, nbins + 1, nullptr, c.scan_scratch, s);
   nb_scatter<<<blocks_for(n, 256), 256, 0, s>>>(n, c.key, c.rank, c.bin_start, c.sorted);
   nb_columns<false><<<1, 1024, 0, s>>>(G.ncol(), G.Nz, nbins, c.bin_start, nullptr, nullptr, c.groups_cap,
@@ -1002,7 +1008,7 @@ static void nb_build_launch(NbCtx &c, const double *x, const double box[3], cuda
 }
 
 void nb_build_launch_public(NbCtx &c, const double *x, const double box[3], cudaStream_t s) {
-  nb_build_launch(c, x, box, s);
+  nb_build_launch(c, x, box, false, s);  // the build of record is the host's last
 }
 
 int nb_reserve_inner(NbCtx &c, cudaStream_t s) {
@@ -1077,12 +1083,13 @@ int nb_build_run(NbCtx &c, const double *x, const double box[3], cudaStream_t s)
   c.plan_bins = G.nbins();
   if (!c.key) {
     if (nb_realloc(c.key, c.n) || nb_realloc(c.sorted, c.n) || nb_realloc(c.atom_xw, c.n) ||
-        nb_realloc(c.atom_shift, c.n) || nb_realloc(c.place_of, c.n) || nb_realloc(c.rank, c.n))
+        nb_realloc(c.atom_shift, c.n) || nb_realloc(c.place_of, c.n) || nb_realloc(c.rank, c.n) ||
+        nb_realloc(c.x_build, 3 * c.n))
       return -1;
   }
   for (int attempt = 0; attempt < 8; ++attempt) {
     if (nb_reserve(c, cap, s)) return -1;
-    nb_build_launch(c, x, box, s);
+    nb_build_launch(c, x, box, true, s);
     NB_CHECK(cudaMemcpyAsync(c.h_sizes, c.sizes, sizeof(int32_t) * NB_SIZE_COUNT,
                              cudaMemcpyDeviceToHost, s));
     NB_CHECK(cudaStreamSynchronize(s));
