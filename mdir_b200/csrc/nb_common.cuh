@@ -115,8 +115,11 @@ __device__ __forceinline__ float3 nb_lattice_shift(int na, int nb, int nc, const
 __device__ __forceinline__ void nb_grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // Lets the chained kernel after this one launch once every block of this
 // grid has called it (or exited): the dependent's blocks then run their work
-// before nb_grid_wait() beside this kernel's.  Called by a persistent kernel
-// whose blocks are all resident, it cannot hold back blocks of its own grid.
+// before nb_grid_wait() beside this kernel's.  Called after this kernel's own
+// nb_grid_wait(), so that what the dependent reads before its wait (of any
+// kernel before this one) is complete and visible.  Called by a persistent
+// kernel whose blocks are all resident, it cannot hold back blocks of its own
+// grid.
 __device__ __forceinline__ void nb_grid_launch_dependents() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }

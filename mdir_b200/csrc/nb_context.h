@@ -309,7 +309,7 @@ void nb_gather_frames(NbCtx &c, const double *x, const double box[3], cudaStream
 // With `skip` (device), nothing when *skip is set (a pruning step whose
 // pairs nb_prune_pairs_run computed).
 // With `update_after`, the kernel lets the chained launch after it (the MD
-// step's update) start beside it once its persistent blocks are resident;
+// step's update) start beside it once its persistent blocks are past their wait;
 // kept off where pair launches follow one another.
 void nb_pairs_run(NbCtx &c, const double box[3], bool energy, cudaStream_t s, const int *halt = nullptr,
                   const int *skip = nullptr, bool update_after = false);

@@ -335,8 +335,9 @@ __global__ void __launch_bounds__(MD_UPDATE_THREADS) md_update(
     int base = 3 * wl, s1 = base + (k + 1) % 3, s2 = base + (k + 2) % 3;
     if (lane >= 30) s1 = s2 = base = lane;
     // every load of data that no kernel of this step writes (the pair
-    // kernel lets this launch start beside it, so the step's pruning may not
-    // have flushed), then the wait
+    // kernel lets this launch start beside it once it is past its own wait:
+    // the update of the step before is complete, the pairs are not), then the
+    // wait
     Vec3 x0 = load3(x, a), v0 = load3(v, a);
     double q = charge[a], im = inv_mass[a], ms = mass[a];
     Vec3 xr = load3(x_ref, a);

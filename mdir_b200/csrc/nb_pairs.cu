@@ -501,10 +501,13 @@ __global__ void __launch_bounds__(NB_PAIR_WARPS * 32, 32 / NB_PAIR_WARPS) nb_pai
                                                 float4 *__restrict__ acc, unsigned long long *__restrict__ accf,
                                                 double *__restrict__ partials, int *__restrict__ status,
                                                 const int *halt, const int *skip) {
-  // the MD step's update may start its loads, its PME gather and its
-  // excluded pairs beside this kernel; it waits for these forces
-  if (P.update_after) nb_grid_launch_dependents();
   nb_grid_wait();  // the lists and frames of the kernels before (a chained launch)
+  // the MD step's update may start its loads, its PME gather and its
+  // excluded pairs beside this kernel; it waits for these forces.  Not before
+  // the wait: the update reads the state that the update of the step before
+  // wrote, and with one list and no reciprocal sum this kernel's wait is all
+  // that stands between the two
+  if (P.update_after) nb_grid_launch_dependents();
   if (halt && *halt) return;  // the MD step stopped at a stale list (its host rebuilds)
   if (skip && *skip) return;  // a pruning step: the pruning kernel computed the pairs
   __shared__ float4 s_x[NB_PAIR_WARPS][2 * NB_GROUP];
