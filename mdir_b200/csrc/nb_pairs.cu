@@ -214,19 +214,15 @@ __device__ __forceinline__ void nb_pair_unit(const PairParams &P, int2 uo, int64
   }
   float ax = 0.f, ay = 0.f, az = 0.f;  // the accumulator of member (lane + k) mod 16
   float elj = 0.f, ecl = 0.f;
-  // The virial sum of d f over the unit's pairs from its sums of forces: each
-  // member's and partner's place, less the group's first, times the force the
-  // unit puts on it (the places lie within the reach of that one, so nothing is
-  // lost to the size of the cell).  Six products an entry instead of six a slot.
+  // The virial, the sum of d f over the unit's pairs.  In the mixed mode from
+  // the unit's sums of forces: each member's and partner's place, less the
+  // group's first, times the force the unit puts on it (six products an entry
+  // instead of six a slot).  A group of a sparse system is long, and the sums'
+  // rounding then counts with its length; the frames' rounding, which counts
+  // with the cell's, hides it.  The deterministic mode's split frames have no
+  // such rounding, so it sums pair by pair.
   float vxx = 0.f, vyy = 0.f, vzz = 0.f, vxy = 0.f, vxz = 0.f, vyz = 0.f;
-  auto virial = [&](float4 x, float3 lo, float fx, float fy, float fz) {
-    const float4 c = s_xw[0];
-    float dx = x.x - c.x, dy = x.y - c.y, dz = x.z - c.z;
-    if (FIXED) {
-      dx += lo.x;
-      dy += lo.y;
-      dz += lo.z;
-    }
+  auto virial = [&](float dx, float dy, float dz, float fx, float fy, float fz) {
     vxx = fmaf(dx, fx, vxx);
     vyy = fmaf(dy, fy, vyy);
     vzz = fmaf(dz, fz, vzz);
@@ -370,6 +366,7 @@ __device__ __forceinline__ void nb_pair_unit(const PairParams &P, int2 uo, int64
       if (ENERGY) {
         elj += inside ? ulj : 0.f;
         ecl += inside ? uc : 0.f;
+        if (FIXED) virial(dx, dy, dz, fx, fy, fz);
       }
     };
     if (__all_sync(FULL, __popc(mask) <= NB_SPARSE_BITS)) {
@@ -434,7 +431,10 @@ __device__ __forceinline__ void nb_pair_unit(const PairParams &P, int2 uo, int64
         az = __shfl_sync(FULL, az, src);
       }
     }
-    if (ENERGY) virial(xj, jl, fjx, fjy, fjz);
+    if (ENERGY && !FIXED) {
+      const float4 c = s_xw[0];
+      virial(xj.x - c.x, xj.y - c.y, xj.z - c.z, fjx, fjy, fjz);
+    }
     if (valid && (fjx != 0.f || fjy != 0.f || fjz != 0.f)) {
       if (FIXED)
         nb_red_fixed(accf + 3 * (int64_t)q, fjx, fjy, fjz, status);
@@ -451,9 +451,9 @@ __device__ __forceinline__ void nb_pair_unit(const PairParams &P, int2 uo, int64
     else
       nb_red_add_v4(acc + pi, ax, ay, az);
   }
-  if (ENERGY && lane < 16) {
-    const float4 lo = FIXED ? s_lw[u] : make_float4(0.f, 0.f, 0.f, 0.f);
-    virial(s_xw[u], make_float3(lo.x, lo.y, lo.z), ax, ay, az);
+  if (ENERGY && !FIXED && lane < 16) {
+    const float4 c = s_xw[0], x = s_xw[u];
+    virial(x.x - c.x, x.y - c.y, x.z - c.z, ax, ay, az);
   }
   if (ENERGY) {
     double v[8] = {elj, ecl, vxx, vyy, vzz, vxy, vxz, vyz};
