@@ -93,58 +93,74 @@ __global__ void nb_scatter(int64_t n, const int32_t *__restrict__ key, const int
   sorted[bin_start[key[i]] + rank[i]] = (int32_t)i;
 }
 
-// The columns' groups, in one block: a thread a column counts its groups of
-// 16 places and a scan gives their first groups, a block's threads of columns
-// at a time (one pass up to 1,024).  Clears the build's sizes and counts the
-// positions with no key (the bin past the grid).  With `frames` (a batch),
-// column c is of frame col_frame[c].
+// The groups of 16 places of column c.  With `frames` (a batch), the column
+// is of frame col_frame[c].
 template <bool BATCH>
-__global__ void __launch_bounds__(1024) nb_columns(int ncol, int Nz, int nbins, const int32_t *__restrict__ bin_start,
+__device__ __forceinline__ int nb_column_groups(int c, int Nz, const int32_t *__restrict__ bin_start,
+                                                const NbFrameDev *__restrict__ frames,
+                                                const int32_t *__restrict__ col_frame) {
+  int b0 = c * Nz, nz = Nz;
+  if (BATCH) {
+    const NbFrameDev &F = frames[col_frame[c]];
+    nz = F.Nz;
+    b0 = F.bin0 + (c - F.col0) * nz;
+  }
+  return (bin_start[b0 + nz] - bin_start[b0] + NB_GROUP - 1) / NB_GROUP;
+}
+
+// The columns' first groups, in one block: a thread a column counts its
+// groups and a scan places them, a block's threads of columns at a time.
+template <bool BATCH>
+__global__ void __launch_bounds__(1024) nb_columns(int ncol, int Nz, const int32_t *__restrict__ bin_start,
                                                    const NbFrameDev *__restrict__ frames,
-                                                   const int32_t *__restrict__ col_frame, int64_t groups_cap,
-                                                   int32_t *__restrict__ group_start, int32_t *__restrict__ sizes) {
+                                                   const int32_t *__restrict__ col_frame,
+                                                   int32_t *__restrict__ group_start) {
   __shared__ int sw[32];
   int before = 0;
   for (int c0 = 0; c0 < ncol; c0 += blockDim.x) {
     const int c = c0 + threadIdx.x;
-    int groups = 0;
-    if (c < ncol) {
-      int b0 = c * Nz, nz = Nz;
-      if (BATCH) {
-        const NbFrameDev &F = frames[col_frame[c]];
-        nz = F.Nz;
-        b0 = F.bin0 + (c - F.col0) * nz;
-      }
-      groups = (bin_start[b0 + nz] - bin_start[b0] + NB_GROUP - 1) / NB_GROUP;
-    }
+    const int groups = c < ncol ? nb_column_groups<BATCH>(c, Nz, bin_start, frames, col_frame) : 0;
     int total;
     const int first = before + nb_block_exclusive_scan(groups, sw, total);
     before += total;
     if (c < ncol) group_start[c] = first;
   }
-  if (threadIdx.x == 0) {
-    group_start[ncol] = before;
-    for (int k = 0; k < NB_SIZE_COUNT; ++k) sizes[k] = 0;
-    sizes[NB_SIZE_GROUPS] = before;
-    sizes[NB_SIZE_PLACES] = before * NB_GROUP;
-    sizes[NB_SIZE_NAN] = bin_start[nbins + 1] - bin_start[nbins];
-    sizes[NB_SIZE_OVERFLOW] = before > groups_cap ? 1 : 0;
-  }
+  if (threadIdx.x == 0) group_start[ncol] = before;
+}
+
+// The columns' groups, a thread a column over the whole GPU (nb_scan places
+// them).
+template <bool BATCH>
+__global__ void nb_column_counts(int ncol, int Nz, const int32_t *__restrict__ bin_start,
+                                 const NbFrameDev *__restrict__ frames, const int32_t *__restrict__ col_frame,
+                                 int32_t *__restrict__ groups) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c < ncol) groups[c] = nb_column_groups<BATCH>(c, Nz, bin_start, frames, col_frame);
 }
 
 // The places, a thread an atom of the bin order: within its bin (half an
 // atom on average) an atom comes after those of a smaller number, so that the
-// order does not depend on the threads.  With `frames`, the columns of a batch.
+// order does not depend on the threads.  Also clears the build's sizes and
+// writes those that the columns give, with the positions that have no key (the
+// bin past the grid).  With `frames`, the columns of a batch.
 template <bool BATCH>
-__global__ void nb_places(int nsorted_max, const int32_t *__restrict__ bin_start, int nvalid_bins,
+__global__ void nb_places(int nsorted_max, int ncol, const int32_t *__restrict__ bin_start, int nvalid_bins,
                           const int32_t *__restrict__ sorted, const int32_t *__restrict__ key, int Nz,
                           const NbFrameDev *__restrict__ frames, const int32_t *__restrict__ atom_frame,
                           const int32_t *__restrict__ group_start, int64_t places_cap,
                           const float4 *__restrict__ atom_xw, const char4 *__restrict__ atom_shift,
                           const int32_t *__restrict__ type, const int32_t *__restrict__ lj_on,
                           int32_t *__restrict__ order, int32_t *__restrict__ place_of,
-                          char4 *__restrict__ shift, float4 *__restrict__ xw) {
+                          char4 *__restrict__ shift, float4 *__restrict__ xw, int32_t *__restrict__ sizes) {
   int s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (s == 0) {
+    const int groups = group_start[ncol];
+    for (int k = 0; k < NB_SIZE_COUNT; ++k) sizes[k] = 0;
+    sizes[NB_SIZE_GROUPS] = groups;
+    sizes[NB_SIZE_PLACES] = groups * NB_GROUP;
+    sizes[NB_SIZE_NAN] = bin_start[nvalid_bins + 1] - bin_start[nvalid_bins];
+    sizes[NB_SIZE_OVERFLOW] = (int64_t)groups * NB_GROUP > places_cap ? 1 : 0;
+  }
   if (s >= nsorted_max) return;
   const int a = sorted[s], k = key[a];
   if (k >= nvalid_bins) {  // positions with no key are in no group
@@ -954,6 +970,26 @@ static void nb_units_run(NbCtx &c, const int32_t *counts, int32_t *unit_start, i
                                                    c.units_cap, unit_start, units, sizes_out, entries, gate, prunes);
 }
 
+// The columns' first groups: one block up to this many columns, above it a
+// count by all of the GPU and a scan, two launches more.  The block's passes of
+// 1,024 columns come one after the other (three dependent loads a column):
+// 6.3 µs for 4,096 columns and 20.3 for 16,384, in a batch 10.1 for 5,500 and
+// 18.7 for 11,000, where the three kernels take 5.3, 8.0, 8.3 and 8.5 beside
+// their launches.
+#define NB_COLUMNS_ONE_BLOCK 8192
+template <bool BATCH>
+static void nb_columns_run(NbCtx &c, int ncol, int Nz, const NbFrameDev *frames, const int32_t *col_frame,
+                           cudaStream_t s) {
+  if (ncol <= NB_COLUMNS_ONE_BLOCK) {
+    nb_columns<BATCH><<<1, 1024, 0, s>>>(ncol, Nz, c.bin_start, frames, col_frame, c.group_start);
+    return;
+  }
+  // the counts of the bins are scanned: their buffer takes the columns' (no
+  // more columns than bins)
+  nb_column_counts<BATCH><<<blocks_for(ncol, 256), 256, 0, s>>>(ncol, Nz, c.bin_start, frames, col_frame, c.bin_count);
+  nb_scan(c.bin_count, c.group_start, ncol, nullptr, c.scan_scratch, s);
+}
+
 // Launches one build on `s`; the sizes are left in c.sizes (device).  The
 // chain is nine launches and two memsets (keys, scan, scatter, columns, places,
 // search, units), two fewer where a block takes a scan alone: the small
@@ -971,12 +1007,11 @@ static void nb_build_launch(NbCtx &c, const double *x, const double box[3], bool
                                             c.bin_count, c.atom_xw, c.atom_shift, keep_x ? c.x_build : nullptr);
   nb_scan(c.bin_count, c.bin_start, nbins + 1, nullptr, c.scan_scratch, s);
   nb_scatter<<<blocks_for(n, 256), 256, 0, s>>>(n, c.key, c.rank, c.bin_start, c.sorted);
-  nb_columns<false><<<1, 1024, 0, s>>>(G.ncol(), G.Nz, nbins, c.bin_start, nullptr, nullptr, c.groups_cap,
-                                       c.group_start, c.sizes);
-  nb_places<false><<<blocks_for(n, 256), 256, 0, s>>>((int)n, c.bin_start, nbins, c.sorted, c.key, G.Nz, nullptr,
+  nb_columns_run<false>(c, G.ncol(), G.Nz, nullptr, nullptr, s);
+  nb_places<false><<<blocks_for(n, 256), 256, 0, s>>>((int)n, G.ncol(), c.bin_start, nbins, c.sorted, c.key, G.Nz, nullptr,
                                                      nullptr, c.group_start, c.places_cap, c.atom_xw, c.atom_shift,
                                                      c.type, nb_lj_order(c) == 1 ? c.lj_on : nullptr, c.order,
-                                                     c.place_of, c.shift, c.xw);
+                                                     c.place_of, c.shift, c.xw, c.sizes);
   SearchParams P;
   P.Lx = (float)box[0];
   P.Ly = (float)box[1];
@@ -1332,14 +1367,13 @@ static void nb_batch_build_launch(mdrtNbBatch &b, const double *x, cudaStream_t 
                                                   c.bin_count, c.atom_xw, c.atom_shift);
   nb_scan(c.bin_count, c.bin_start, nbins + 1, nullptr, c.scan_scratch, s);
   nb_scatter<<<blocks_for(n, 256), 256, 0, s>>>(n, c.key, c.rank, c.bin_start, c.sorted);
-  nb_columns<true><<<1, 1024, 0, s>>>(ncol, 1, nbins, c.bin_start, b.frames_dev, b.col_frame, c.groups_cap,
-                                      c.group_start, c.sizes);
+  nb_columns_run<true>(c, ncol, 1, b.frames_dev, b.col_frame, s);
   nb_batch_group_frames<<<blocks_for(ncol, 128), 128, 0, s>>>(ncol, c.group_start, c.groups_cap, b.col_frame,
                                                              b.frames_dev, b.group_frame, b.group_L);
-  nb_places<true><<<blocks_for(n, 256), 256, 0, s>>>((int)n, c.bin_start, nbins, c.sorted, c.key, 1, b.frames_dev,
+  nb_places<true><<<blocks_for(n, 256), 256, 0, s>>>((int)n, ncol, c.bin_start, nbins, c.sorted, c.key, 1, b.frames_dev,
                                                     b.atom_frame, c.group_start, c.places_cap, c.atom_xw,
                                                     c.atom_shift, c.type, nb_lj_order(c) == 1 ? c.lj_on : nullptr,
-                                                    c.order, c.place_of, c.shift, c.xw);
+                                                    c.order, c.place_of, c.shift, c.xw, c.sizes);
   SearchParams P = {};
   P.groups_cap = c.groups_cap;
   P.list_cap = c.list_cap;
