@@ -448,6 +448,29 @@ int32_t mdrtNbSetDeterministic(mdrtNb *ctx, int32_t on) {
   return MDRT_NB_OK;
 }
 
+// Atoms from which a force call's reciprocal chain runs beside its pairs: the
+// fork and join cost the host about 4 µs a call, which a small system, bound
+// by its launches, does not get back (3,000 atoms: 39 µs a call with one
+// stream, 43 with two; 8,013: 61 and 51; 23,550: 64 and 54).  With energies the
+// pairs' branch is longer (their sums): 3,000 atoms 64 and 52 µs.
+#define NB_BESIDE_ATOMS 6000
+#define NB_BESIDE_ENERGY_ATOMS 2000
+static bool nb_beside(const NbCtx &c, bool energy) {
+  return c.pme.on && c.beta > 0.0 && c.n >= (energy ? NB_BESIDE_ENERGY_ATOMS : NB_BESIDE_ATOMS);
+}
+
+// The stream and the events of that fork, made by the first build (or the
+// reciprocal sum set after it) of a context that can use them; any other's
+// would lengthen its first evaluation for nothing.
+static cudaError_t nb_side_stream(mdrtNb *ctx) {
+  int least = 0, greatest = 0;
+  cudaError_t e = cudaDeviceGetStreamPriorityRange(&least, &greatest);
+  if (e == cudaSuccess && !ctx->ev_fork) e = cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming);
+  if (e == cudaSuccess && !ctx->ev_join) e = cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming);
+  if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&ctx->side, cudaStreamNonBlocking, greatest);
+  return e;
+}
+
 int32_t mdrtPmeSetup(mdrtNb *ctx, int32_t k1, int32_t k2, int32_t k3, int32_t order) {
   if (!ctx) return MDRT_NB_INVALID_ARGUMENT;
   NbCtx &c = ctx->c;
@@ -460,6 +483,7 @@ int32_t mdrtPmeSetup(mdrtNb *ctx, int32_t k1, int32_t k2, int32_t k3, int32_t or
   int s = nb_pme_setup(c, k1, k2, k3, order);
   if (s == -2) return MDRT_NB_UNSUPPORTED;
   if (s != 0) return MDRT_NB_CUDA_ERROR;
+  if (c.built && !ctx->side && nb_beside(c, true)) CK(nb_side_stream(ctx));
   return MDRT_NB_OK;
 }
 
@@ -510,13 +534,7 @@ static int32_t nb_build_entry(mdrtNb *ctx, const double *x, int64_t n, const dou
   cudaStream_t st = (cudaStream_t)stream;
   if (nb_build_run(c, x, box, st)) return MDRT_NB_CUDA_ERROR;
   for (int k = 0; k < 3; ++k) c.tilt_built[k] = c.tilt[k];
-  if (!ctx->side) {
-    int least = 0, greatest = 0;
-    CK(cudaDeviceGetStreamPriorityRange(&least, &greatest));
-    CK(cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming));
-    CK(cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming));
-    CK(cudaStreamCreateWithPriority(&ctx->side, cudaStreamNonBlocking, greatest));
-  }
+  if (!ctx->side && nb_beside(c, true)) CK(nb_side_stream(ctx));
   if (sizes_out)
     for (int k = 0; k < NB_SIZE_COUNT; ++k) sizes_out[k] = c.h_sizes[k];
   if (c.h_sizes[NB_SIZE_NAN] > 0) return MDRT_NB_NAN_POSITION;
@@ -543,14 +561,6 @@ int32_t mdrtNbForceTriclinic(mdrtNb *ctx, const double *x, const double cell[6],
   return nb_force_entry(ctx, x, cell, flags, forces, stream, true);
 }
 
-// Atoms from which a force call's reciprocal chain runs beside its pairs: the
-// fork and join cost the host about 4 µs a call, which a small system, bound
-// by its launches, does not get back (3,000 atoms: 39 µs a call with one
-// stream, 43 with two; 8,013: 61 and 51; 23,550: 64 and 54).  With energies the
-// pairs' branch is longer (their sums): 3,000 atoms 64 and 52 µs.
-#define NB_BESIDE_ATOMS 6000
-#define NB_BESIDE_ENERGY_ATOMS 2000
-
 // `beside`: the reciprocal chain on the context's own stream beside the
 // pairs (the frames entries keep one stream a lane: their lanes fill the GPU).
 static int32_t nb_force_entry(mdrtNb *ctx, const double *x, const double box[3], uint32_t flags, double *forces,
@@ -570,7 +580,7 @@ static int32_t nb_force_entry(mdrtNb *ctx, const double *x, const double box[3],
   nb_gather_frames(c, x, box, st);
   const bool gathers = pme && nb_finish_gathers(c);
   const bool potential = (flags & MDRT_NB_POTENTIAL) != 0;
-  beside = beside && pme && pairs && ctx->side && c.n >= (energy ? NB_BESIDE_ENERGY_ATOMS : NB_BESIDE_ATOMS);
+  beside = beside && pme && pairs && ctx->side && nb_beside(c, energy);
   if (beside) {
     CK(cudaEventRecord(ctx->ev_fork, st));
     CK(cudaStreamWaitEvent(ctx->side, ctx->ev_fork, 0));

@@ -98,3 +98,32 @@ def test_calls_captured_in_a_graph_replay(cuda):
         torch.cuda.synchronize()
         assert torch.equal(out, want[-1])  # fixed-point sums: the same bits
     t.close()
+
+
+@pytest.mark.parametrize("waters", [600, 2200])  # without and with a stream of its own for the chain
+def test_a_first_call_in_a_graph_and_a_sum_set_after_the_build(cuda, waters):
+    from mdir_b200 import systems
+    s = systems.tip3p(waters=waters, seed=2)
+    x = torch.tensor(s["positions"], device=cuda)
+    t = term(s, 4, True)
+    t.build(x, s["box"])
+    t.force(x, energy=True)
+    want = t.force(x).clone()  # fixed-point sums: the same bits on every route
+    late = term(s, 4, True)
+    late.set_pme((0, 0, 0), 4)
+    late.build(x, s["box"])
+    late.set_pme(s["grid"], 4)
+    assert torch.equal(late.force(x), want)
+    first = term(s, 4, True)
+    first.build(x, s["box"])
+    out = torch.empty_like(x)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        first.force(x, forces=out)
+    for _ in range(2):
+        out.zero_()
+        g.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, want)
+    for k in (t, late, first):
+        k.close()
