@@ -581,15 +581,26 @@ static int32_t nb_force_entry(mdrtNb *ctx, const double *x, const double box[3],
   const bool gathers = pme && nb_finish_gathers(c);
   const bool potential = (flags & MDRT_NB_POTENTIAL) != 0;
   beside = beside && pme && pairs && ctx->side && nb_beside(c, energy);
+  // joins the chain where the forces are finished, or where an error returns
+  struct Join {
+    cudaStream_t st = nullptr, side = nullptr;
+    cudaEvent_t done = nullptr;
+    cudaError_t operator()() {
+      if (!side) return cudaSuccess;
+      cudaError_t e = cudaEventRecord(done, side);
+      if (e == cudaSuccess) e = cudaStreamWaitEvent(st, done, 0);
+      side = nullptr;
+      return e;
+    }
+    ~Join() { (*this)(); }
+  } join;
   if (beside) {
     CK(cudaEventRecord(ctx->ev_fork, st));
     CK(cudaStreamWaitEvent(ctx->side, ctx->ev_fork, 0));
-    const int rc = nb_pme_run(c, box, energy, potential, ctx->side, !gathers);
-    CK(cudaEventRecord(ctx->ev_join, ctx->side));  // joined below, also after an error
-    if (rc) {
-      CK(cudaStreamWaitEvent(st, ctx->ev_join, 0));
-      return MDRT_NB_CUDA_ERROR;
-    }
+    join.st = st;
+    join.side = ctx->side;
+    join.done = ctx->ev_join;
+    if (nb_pme_run(c, box, energy, potential, ctx->side, !gathers)) return MDRT_NB_CUDA_ERROR;
   }
   bool pairs_done = false;
   if ((flags & MDRT_NB_PRUNE) && c.inner_reach > 0.0) {
@@ -614,7 +625,7 @@ static int32_t nb_force_entry(mdrtNb *ctx, const double *x, const double box[3],
   if (excluded) nb_excluded_run(c, box, energy, st);
   if (energy && (pairs || excluded)) nb_reduce_energy(c, pairs, excluded, st);
   if (beside) {
-    CK(cudaStreamWaitEvent(st, ctx->ev_join, 0));
+    CK(join());
   } else if (pme) {
     if (nb_pme_run(c, box, energy, potential, st, !gathers)) return MDRT_NB_CUDA_ERROR;
   }

@@ -1384,6 +1384,13 @@ int nb_pme_run(NbCtx &c, const double box[3], bool energy, bool potential, cudaS
   nb_cell_tilts(c, box, G, nullptr);
   int64_t total = (int64_t)G.K0 * G.K1 * G.K2;
   int64_t half = (int64_t)G.K0 * G.K1 * (G.K2 / 2 + 1);
+  if (!energy && nb_pme_table(c, box, s)) return -1;
+  // the grid is empty between calls: one that fails after the spreading clears it
+  auto fail = [&]() {
+    cudaMemsetAsync(P.grid, 0, sizeof(float) * total, s);
+    cudaMemsetAsync(P.fixed, 0, sizeof(unsigned long long) * total, s);
+    return -3;
+  };
   nb_spread_run(c, G, P.grid, P.fixed, nullptr, s);
   bool own = nb_fft_own(c);
   if (c.deterministic && !own) nb_fixed_to_grid<<<blocks_for((total + 3) / 4, 256), 256, 0, s>>>(total, P.fixed, P.grid);
@@ -1401,24 +1408,22 @@ int nb_pme_run(NbCtx &c, const double box[3], bool energy, bool potential, cudaS
   if (own) {
     // spread grid -> potential, the fixed-point grid read directly; the grid it
     // read is empty again
-    if (!energy && nb_pme_table(c, box, s)) return -1;
     if (nb_fft_convolve(P, P.grid, c.deterministic ? P.fixed : nullptr, P.spec, P.phi, P.influence, energy, C,
                         P.partials, nullptr, s))
-      return -3;
+      return fail();
     if (energy) nb_pme_sums(c, (int)nb_fft_column_blocks(P.K), s);
   } else {
     cufftSetStream(P.fwd, s);
     cufftSetStream(P.bwd, s);
-    if (cufftExecR2C(P.fwd, P.grid, (cufftComplex *)P.spec) != CUFFT_SUCCESS) return -3;
+    if (cufftExecR2C(P.fwd, P.grid, (cufftComplex *)P.spec) != CUFFT_SUCCESS) return fail();
     if (energy) {
       nb_convolve<true><<<blocks_for(half, 256), 256, 0, s>>>(C, P.moduli, P.spec, P.partials);
       cudaMemsetAsync(P.grid, 0, sizeof(float) * total, s);  // empty for the next spreading
       nb_pme_sums(c, P.conv_blocks, s);
     } else {
-      if (nb_pme_table(c, box, s)) return -1;
       nb_scale_spectrum<<<blocks_for(half, 256), 256, 0, s>>>(half, P.influence, P.spec, P.grid, total, nullptr);
     }
-    if (cufftExecC2R(P.bwd, (cufftComplex *)P.spec, P.phi) != CUFFT_SUCCESS) return -3;
+    if (cufftExecC2R(P.bwd, (cufftComplex *)P.spec, P.phi) != CUFFT_SUCCESS) return fail();
   }
   if (!gather) return 0;
   float *pot = potential ? P.potential : nullptr;
