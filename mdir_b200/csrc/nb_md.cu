@@ -96,11 +96,7 @@ struct mdrtMd {
   // graph
   cudaGraphExec_t exec = nullptr;
   cudaGraph_t graph = nullptr;
-  const double *gx = nullptr, *gv = nullptr;
-  double gbox[3] = {0, 0, 0};
-  double gdt = 0.0;
-  int gunroll = 0;
-  int64_t gcap_key = -1;
+  std::vector<uint64_t> gkey;      // what its launches were captured from (md_graph_key)
   std::vector<cudaGraphConditionalHandle> handles;
 };
 
@@ -735,8 +731,8 @@ static int32_t *md_unit_counter(mdrtMd &m) {
 }
 
 // The pruning of a step when the update before it asked for it (flag[1],
-// on the device): one launch (two in the deterministic mode) that does
-// nothing otherwise, no conditional node.
+// on the device): one launch (in the deterministic mode two, three for more
+// than 4,096 groups) that does nothing otherwise, no conditional node.
 static void md_prune_step(mdrtMd &m, const double *x, const double box[3], cudaStream_t s) {
   NbCtx &c = *m.nb;
   if (c.inner_reach > 0.0)
@@ -1236,18 +1232,42 @@ static int32_t md_restore(mdrtMd *m, double *x, double *v, const double box[3], 
   return MDRT_NB_OK;
 }
 
+// What the launches of a step graph take from the context and the call: the
+// graph serves while all of it is as it was at the capture.  (The thermostat,
+// the look-ahead and the integrator's own buffers drop the graph themselves.)
+static std::vector<uint64_t> md_graph_key(const mdrtMd &m, const double *x, const double *v, const double box[3],
+                                          double dt, int32_t unroll) {
+  const NbCtx &c = *m.nb;
+  const NbPme &p = c.pme;
+  std::vector<uint64_t> key;
+  for (double d : {box[0], box[1], box[2], dt, c.cutoff, c.reach, c.inner_reach, c.beta, c.coulomb,
+                   c.switch_distance}) {
+    uint64_t bits;
+    std::memcpy(&bits, &d, sizeof(bits));
+    key.push_back(bits);
+  }
+  for (int64_t k : {(int64_t)unroll, c.groups_cap, c.list_cap, c.units_cap, c.bins_cap, (int64_t)c.inner_valid,
+                    (int64_t)c.deterministic, (int64_t)c.pair_blocks_per_sm, (int64_t)c.pair_sms,
+                    (int64_t)nb_fused_prune(c), (int64_t)c.staging_depth, (int64_t)nb_fft_own(c),
+                    (int64_t)nb_pme_tiled(c), (int64_t)c.coulomb_shift, (int64_t)c.lj_switch, (int64_t)c.ntypes,
+                    (int64_t)c.lj_geom, (int64_t)c.lj_mask, (int64_t)p.on, (int64_t)p.order, (int64_t)p.K[0],
+                    (int64_t)p.K[1], (int64_t)p.K[2]})
+    key.push_back((uint64_t)k);
+  for (const void *q : {(const void *)x, (const void *)v, (const void *)c.slab, (const void *)c.slab_in,
+                        (const void *)c.units, (const void *)c.units_in, (const void *)c.xq, (const void *)c.acc,
+                        (const void *)c.bin_count, (const void *)c.scan_scratch, (const void *)c.group_start,
+                        (const void *)c.excl_off, (const void *)c.excl, (const void *)c.excl_pairs,
+                        (const void *)p.grid, (const void *)p.fft_tw, (const void *)p.pme_force, (const void *)m.qgrid,
+                        (const void *)m.phi, (const void *)m.spec, (const void *)m.influence})
+    key.push_back((uint64_t)(uintptr_t)q);
+  return key;
+}
+
 // The graph of `unroll` steps (gated prunings, one conditional rebuild at
-// the end), captured again when its arguments or the capacities changed.
+// the end), captured again when what it was captured from changed.
 static int32_t md_prepare_graph(mdrtMd *m, double *x, double *v, const double box[3], double dt, int32_t unroll) {
-  NbCtx &c = *m->nb;
-  int64_t key = c.groups_cap * 1000003 + c.list_cap * 7 + c.units_cap + (int64_t)(c.inner_reach * 1e9) +
-                (c.inner_valid ? 1 : 0) + (c.deterministic ? 2 : 0) + ((int64_t)c.pair_blocks_per_sm << 40) +
-                ((int64_t)c.pair_sms << 44) + (int64_t)(uintptr_t)m->qgrid + ((int64_t)nb_fused_prune(c) << 56) +
-                ((int64_t)c.staging_depth << 58) + ((int64_t)nb_fft_own(c) << 61) +
-                ((int64_t)nb_pme_tiled(c) << 62);
-  bool stale = !m->exec || m->gx != x || m->gv != v || m->gdt != dt || m->gunroll != unroll ||
-               m->gbox[0] != box[0] || m->gbox[1] != box[1] || m->gbox[2] != box[2] || m->gcap_key != key;
-  if (stale) {
+  std::vector<uint64_t> key = md_graph_key(*m, x, v, box, dt, unroll);
+  if (!m->exec || m->gkey != key) {
     md_drop_graph(m);
     // A window of `unroll` steps: each step prunes when its update asks
     // (gated launches, no conditional node), and the last step decides the
@@ -1290,12 +1310,7 @@ static int32_t md_prepare_graph(mdrtMd *m, double *x, double *v, const double bo
       return MDRT_NB_CUDA_ERROR;
     }
     m->graph = graph;
-    m->gx = x;
-    m->gv = v;
-    m->gdt = dt;
-    m->gunroll = unroll;
-    m->gcap_key = key;
-    for (int k = 0; k < 3; ++k) m->gbox[k] = box[k];
+    m->gkey = std::move(key);
   }
   return MDRT_NB_OK;
 }
