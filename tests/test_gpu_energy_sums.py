@@ -40,15 +40,53 @@ def test_energies_are_the_oracles_and_reproducible(cuda, waters):
         assert abs(value - ref[k]) <= 1e-6 * scale
 
 
-def test_batch_constants_follow_the_charges(cuda):
-    from mdir_b200 import systems
+def test_constants_follow_the_charges_set_again(cuda):
+    """The sums of the charges are kept where they are set: a second set of
+    charges (here of a net charge of 0.8 a system) replaces them, in a batch and
+    in a context, in the constants and in the energy gradient's background."""
+    from mdir_b200 import NonbondedTerm, systems
+    from mdir_b200 import _lib as L
     from mdir_b200.batch import BatchEvaluator
+    from mdir_b200.term import _hp
     frames = systems.batch_frames(count=5, low=1000, high=2000, seed=8)
+
+    def wanted(f, q):
+        V = float(np.prod(f["box"]))
+        return (-systems.COULOMB * f["beta"] / np.sqrt(np.pi) * np.sum(q * q),
+                -systems.COULOMB * np.pi * np.sum(q) ** 2 / (2 * V * f["beta"] ** 2))
+
     ev = BatchEvaluator(frames)
-    ev.force(energy=True)
-    e = ev.energies()
-    for k, f in enumerate(frames):
-        q = np.asarray(f["charges"])
-        want = -systems.COULOMB * f["beta"] / np.sqrt(np.pi) * np.sum(q * q)
-        assert abs(e["self"][k] - want) <= 1e-12 * abs(want)
+    old = [np.asarray(f["charges"]) for f in frames]
+    new = [1.1 * q + 0.8 / len(q) for q in old]
+    types = np.ascontiguousarray(np.concatenate([f["types"] for f in frames]), dtype=np.int32)
+    sigma, epsilon = (np.ascontiguousarray(frames[0][k], dtype=np.float64) for k in ("sigma", "epsilon"))
+    for charges in (old, new, old):
+        q = np.ascontiguousarray(np.concatenate(charges), dtype=np.float64)
+        L.check(L.lib().mdrtNbBatchSetParticles(ev._h, _hp(q), _hp(types), len(sigma), _hp(sigma), _hp(epsilon)),
+                "mdrtNbBatchSetParticles")
+        ev.force(energy=True)
+        e = ev.energies()
+        for k, (f, q) in enumerate(zip(frames, charges)):
+            for got, want in zip((e["self"][k], e["background"][k]), wanted(f, q)):
+                assert abs(got - want) <= 1e-12 * abs(want) + 1e-15, (k, got, want)
     ev.close()
+    f, q0, q1 = frames[0], old[0], new[0]
+    x = torch.tensor(f["positions"], device=cuda)
+
+    seen = []
+    for sequence in ((q0, q1), (q1,)):
+        t = NonbondedTerm(len(q0))
+        t.set_exclusions(pairs=f["excluded_pairs"])
+        t.set_interaction(f["cutoff"], f["reach"], f["beta"])
+        t.set_pme(f["grid"], f["order"])
+        for q in sequence:
+            t.set_particles(q, f["types"], f["sigma"], f["epsilon"])
+            t.build(x, f["box"])
+            c = t.constants(f["box"])
+            for got, want in zip((c["self"], c["background"]), wanted(f, q)):
+                assert abs(got - want) <= 1e-12 * abs(want) + 1e-15
+            dq, _ = t.parameter_gradient(x)
+        seen.append(dq)
+        t.close()
+    # f32 pair terms summed by atomics in two orders: 1e-6 of the norm
+    assert float((seen[0] - seen[1]).norm()) <= 1e-6 * float(seen[1].norm())

@@ -88,7 +88,7 @@ def test_large_lists_hold_every_pair(cuda, n, tilts):
     assert have <= key(free(near(x, cell, R + wide + 1e-5)))
 
 
-def test_one_and_four_warps_a_group_give_the_same_lists(cuda):
+def test_lists_of_one_and_four_warps_a_group_sum_to_the_same_bits(cuda):
     from mdir_b200 import systems
     from mdir_b200.batch import BatchEvaluator
     frames = systems.batch_frames(count=7, low=1000, high=4000, seed=11)
@@ -100,7 +100,8 @@ def test_one_and_four_warps_a_group_give_the_same_lists(cuda):
         ev.force(energy=True)
         lists.append(ev.energies())
         ev.close()
-    # the same lists entry for entry: the pair energies, summed unit by unit, are the same bits
+    # a batch shows no lists; a unit's energies and virial are f32 sums over its
+    # entries in their order, so that another entry or order would change bits
     for term in ("lj", "coulomb"):
         np.testing.assert_array_equal(lists[0][term], lists[1][term])
 
