@@ -379,9 +379,10 @@ int32_t mdrtNbStatus(mdrtNb *ctx, void *stream, int32_t clear, int32_t *status);
 /* Average device time (ms, CUDA events on `stream`) of `iterations`
  * launches of each stage of the force term at device positions x, after a
  * valid build: out[0] frame gather, out[1] pair kernel, out[2] excluded
- * correction, out[3] PME (spread, FFTs, convolution, gather), out[4] force
- * finish, out[5] neighbor build (launches only), out[6] pruning (0 without
- * a dual list); out holds 8 doubles.  The launches of a stage are replayed
+ * correction, out[3] PME (spread, FFTs, convolution; the gather at orders 5
+ * and 6), out[4] force finish (with the PME gather at orders 4 and 8),
+ * out[5] neighbor build (launches only), out[6] pruning (0 without a dual
+ * list); out holds 8 doubles.  The launches of a stage are replayed
  * from a CUDA graph, so the host's launch rate does not enter the numbers.
  * For the roofline of each kernel; the forces it leaves are not meaningful.
  * MDIR: MDRT_WAIT=1 per-kernel timing (runtime/mdrt_cuda.c:600). */

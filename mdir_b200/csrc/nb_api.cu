@@ -71,8 +71,9 @@ __global__ void nb_frame_drift(int64_t n, const double *__restrict__ frames, con
 // build count of NbCtx, so that any change of the context that alters what
 // the launches are (a build, a growth, new tuning, a new cell) changes the
 // key.  The graph reads the frames, the particle tables and the lists at its
-// launch.  The host arrays of NbCtx (h_q and the like) are not in the key:
-// the launches kept here take no argument computed from them.
+// launch.  What the host arrays of NbCtx hold (h_type and the like) and
+// the charge sums of mdrtNb are not in the key: the launches kept here take no
+// argument computed from them.
 #define NB_FRAME_GRAPHS 8
 
 std::vector<unsigned char> nb_frames_key(const NbCtx &c, const uint64_t *args, int nargs) {
@@ -255,11 +256,10 @@ int32_t mdrtNbSetParticles(mdrtNb *ctx, const double *charges, const int32_t *ty
   CK(cudaSetDevice(c.device));
   for (int64_t i = 0; i < c.n; ++i)
     if (types[i] < 0 || types[i] >= ntypes || !std::isfinite(charges[i])) return MDRT_NB_INVALID_ARGUMENT;
-  c.h_q.assign(charges, charges + c.n);
   ctx->q_sum = ctx->q_sq = 0.0;
-  for (double v : c.h_q) {
-    ctx->q_sq += v * v;
-    ctx->q_sum += v;
+  for (int64_t i = 0; i < c.n; ++i) {
+    ctx->q_sq += charges[i] * charges[i];
+    ctx->q_sum += charges[i];
   }
   const bool same_types = (int64_t)c.h_type.size() == c.n && std::equal(c.h_type.begin(), c.h_type.end(), types);
   c.h_type.assign(types, types + c.n);
@@ -1000,8 +1000,15 @@ extern "C" int32_t mdrtNbTimeKernels(mdrtNb *ctx, const double *x, const double 
   out[0] = timed([&] { nb_gather_frames(c, x, box, st); });
   out[1] = timed([&] { nb_pairs_run(c, box, false, st); });
   out[2] = timed([&] { nb_excluded_run(c, box, false, st); });
-  out[3] = (c.pme.on && c.beta > 0) ? timed([&] { nb_pme_run(c, box, false, false, st); }) : 0.0;
-  out[4] = timed([&] { nb_finish_forces(c, scratch, 0, st); });
+  // the chain and the finish as a force call launches them
+  const bool pme = c.pme.on && c.beta > 0, gathers = pme && nb_finish_gathers(c);
+  out[3] = pme ? timed([&] { nb_pme_run(c, box, false, false, st, !gathers); }) : 0.0;
+  out[4] = timed([&] {
+    if (gathers)
+      nb_finish_gather_run(c, box, scratch, 0, false, st);
+    else
+      nb_finish_forces(c, scratch, 0, st);
+  });
   // the neighbor build with its present capacities (no host wait) and the
   // pruning; the lists they leave are those of x again
   out[5] = timed([&] { nb_build_launch_public(c, x, box, st); });

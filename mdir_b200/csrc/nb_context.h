@@ -59,7 +59,6 @@ struct NbCtx {
   float2 *lj = nullptr;  // (c6, c12) per type pair, c6 = 4 eps sig^6, c12 = 4 eps sig^12
   float2 *ljf = nullptr;  // per type (sqrt c6, sqrt c12) when the table factorizes
   bool lj_geom = false;   // c6_ab = f_a f_b and c12_ab = g_a g_b for every pair of types
-  std::vector<double> h_q;     // f64 charges for the host constants
   std::vector<double> h_c6;    // f64 c6 = 4 eps sig^6 per type pair
   std::vector<int32_t> h_type;
   std::vector<float2> h_lj;
@@ -191,7 +190,7 @@ struct mdrtNb {
   std::vector<NbFrameGraph> graphs;
   uint64_t graph_clock = 0;
   // the sums of the charges and of their squares, in atom order, as the
-  // particles were set; kept out of NbCtx like the charges themselves
+  // particles were set; kept out of NbCtx, whose bytes key the frames graphs
   double q_sum = 0.0, q_sq = 0.0;
   // the reciprocal chain of a force call runs on `side` beside its pairs
   cudaStream_t side = nullptr;
@@ -283,10 +282,12 @@ void nb_build_launch_public(NbCtx &c, const double *x, const double box[3], cuda
 // The pruning of the outer lists into the inner ones at the current frames
 // xq (gathered by the caller), and the inner units; no host wait.
 void nb_prune_run(NbCtx &c, const double box[3], cudaStream_t s);
-// The same pruning as two launches that do nothing unless *gate (device) is
-// set: the inner lists with the positions of the pruning copied to x_prune,
-// then the inner units in one block, counting the pruning in *prunes.  The
-// per-step pruning of the MD step, which needs no conditional node.
+// The same pruning as launches that do nothing unless *gate (device) is set:
+// the inner lists with the positions of the pruning copied to x_prune, whose
+// blocks claim their units from unit_counter and count the pruning in *prunes,
+// or without one (the deterministic mode) one or two launches more for the
+// inner units in group order.  The per-step pruning of the MD step, which needs
+// no conditional node.
 void nb_prune_gated(NbCtx &c, const double box[3], const int *gate, const double *x, double *x_prune,
                     double *prunes, int32_t *unit_counter, cudaStream_t s);
 // Allocates the inner lists to the outer capacities (host, between launches);
