@@ -52,7 +52,8 @@ class Integrator:
         L.check(L.lib().mdrtMdSetIntegrator(self._h, code), "mdrtMdSetIntegrator")
 
     def lookahead(self, factor):
-        """The rebuild decision's extrapolation of the drift (default 1.5)."""
+        """The rebuild decision's extrapolation of the drift (default 1.5;
+        two thirds of it after the first window of a build)."""
         L.check(L.lib().mdrtMdSetLookahead(self._h, float(factor)), "mdrtMdSetLookahead")
 
     def build(self, x, box, stream=None):
