@@ -627,7 +627,12 @@ static int32_t nb_force_entry(mdrtNb *ctx, const double *x, const double box[3],
   if (beside) {
     CK(join());
   } else if (pme) {
-    if (nb_pme_run(c, box, energy, potential, st, !gathers)) return MDRT_NB_CUDA_ERROR;
+    if (nb_pme_run(c, box, energy, potential, st, !gathers)) {
+      // the accumulators are empty between calls: no finish empties them here
+      cudaMemsetAsync(c.acc, 0, sizeof(float4) * c.places_cap, st);
+      cudaMemsetAsync(c.acc_fixed, 0, sizeof(unsigned long long) * 3 * c.places_cap, st);
+      return MDRT_NB_CUDA_ERROR;
+    }
   }
   const int accumulate = flags & MDRT_NB_ACCUMULATE ? 1 : 0;
   if (gathers) {

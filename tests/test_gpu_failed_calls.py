@@ -1,7 +1,7 @@
-"""A force call that fails after its charges were spread leaves no charge
-behind: the call after it gives the forces of a fresh context.  The failure is
-made on the host, by a library preloaded before cuFFT whose execution entry
-returns an error once."""
+"""A force call that fails after its charges were spread leaves no charge and
+no pair force behind: the call after it gives the forces of a fresh context.
+The failure is made on the host, by a library preloaded before cuFFT whose
+execution entry returns an error once."""
 
 import os
 import subprocess
@@ -34,7 +34,6 @@ from mdir_b200 import NonbondedTerm, systems
 from mdir_b200._lib import NativeError
 shim = ctypes.CDLL(os.environ["LD_PRELOAD"])
 deterministic, waters = sys.argv[1] == "1", int(sys.argv[2])
-beside = waters > 2000  # the chain beside the pairs, which are launched after it
 s = systems.tip3p(waters=waters, seed=2)
 x = torch.tensor(s["positions"], device="cuda")
 t = NonbondedTerm(len(s["charges"]))
@@ -46,17 +45,17 @@ t.set_tuning(pme_fft="cufft")
 t.set_deterministic(deterministic)
 t.build(x, s["box"])
 for energy in (False, True):
-    want = t.force(x, energy=energy, pairs=False, excluded=False).clone()
+    want = t.force(x, energy=energy).clone()
     for entry in ("fail_r2c", "fail_c2r"):
         ctypes.c_int.in_dll(shim, entry).value = 1
         try:
-            t.force(x, energy=energy, pairs=beside, excluded=False)
+            t.force(x, energy=energy)
             raise SystemExit("the call did not fail")
         except NativeError:
             pass
         assert ctypes.c_int.in_dll(shim, entry).value == 0
-        got = t.force(x, energy=energy, pairs=False, excluded=False)
-        # f32 sums in another order at most: 2e-6 of the norm (a grid with twice the charge: 1)
+        got = t.force(x, energy=energy)
+        # f32 sums in another order at most: 2e-6 of the norm (twice the pairs' forces or the charges: some 0.1 to 1)
         off = float((got - want).norm() / want.norm())
         assert off <= 2e-6, (entry, energy, off)
 print("as a fresh context's")
