@@ -347,7 +347,7 @@ int32_t mdrtNbBatchAutotune(mdrtNbBatch *b, const double *x, double *forces, voi
   CK(cudaEventCreate(&e0));
   CK(cudaEventCreate(&e1));
   float best = 1e30f;
-  int best_w = 4, best_p = c.pair_blocks_per_sm, best_d = c.staging_depth;
+  int best_w = b->search_warps, best_p = c.pair_blocks_per_sm, best_d = c.staging_depth;
   int32_t status = MDRT_NB_OK;
   for (int w : {4, 1}) {
     for (int trial = 0; trial < 8; ++trial) {
